@@ -564,34 +564,14 @@ __global__ void splitGroupsKernel(const uint32_t* failed, uint32_t numFailed, co
     if (sys) newSys[slot] = newSys[slot + 1] = sys[g];
 }
 
-/*! run a traversal to completion: groups that overflow the stack are split in two along the SFC and traversed
- *  again until none fails (traversal_gpu.cu:572-623); counts per group refer to the groups of @p t */
-/*! the interaction count (direct bodies + 2 x approximated cells) past which a group is taken off its warp and
- *  split over several in a second pass. Uniform and Plummer groups stay well below it (at most about 17,000 at theta
- *  0.5); the groups that pass it are sparse outskirts whose bounding box reaches the dense centre, with up to a few
- *  hundred thousand direct bodies, which one warp would evaluate while the rest of the GPU idles. */
-constexpr unsigned kHeavyCost      = 32768;
-constexpr unsigned kWarpSlotsPerSm = 20;   // resident traversal warps per SM (5 blocks of 4)
-constexpr unsigned kGroupsPerSlot  = 4;    // groups per warp slot from which a launch balances by itself
-constexpr unsigned kMinHeavyCost   = 1024; // 16 evaluation batches
-
-/*! the split threshold of a solve of @p numGroups groups. A solve with several groups per warp slot balances by
- *  itself and keeps kHeavyCost. A smaller one (a small system, or the last requests of a served stream) is bound by
- *  its slowest warps, so its threshold falls in proportion to its group count and more of its groups are spread
- *  over several warps: a 2^14-body Plummer sphere traverses in 0.38 ms instead of 0.86 ms. */
-unsigned heavyCostFor(uint32_t numGroups, int smCount)
-{
-    const uint64_t full = uint64_t(smCount) * kWarpSlotsPerSm * kGroupsPerSlot;
-    if (numGroups >= full) return kHeavyCost;
-    return unsigned(std::max<uint64_t>(kMinHeavyCost, uint64_t(kHeavyCost) * numGroups / full));
-}
-
-//! warps per queued group: enough items to fill the GPU, at most 16 (each part repeats the group's walk)
-int heavyParts(uint32_t numHeavy, int smCount)
-{
-    uint32_t want = (uint32_t(smCount) * kWarpSlotsPerSm + numHeavy - 1) / numHeavy;
-    return int(std::max(2u, std::min(16u, want)));
-}
+/*! groups up to which a traversal goes through interaction lists: walks first, then the evaluation of list pieces of
+ *  similar cost by all warps. Larger ones keep the GPU busy with a group per warp, which saves the lists' traffic. */
+constexpr uint32_t kListGroups  = 49152;
+constexpr uint32_t kSubGroups   = 6000;  // groups up to which every list walk is split into eight parts
+constexpr size_t kListBytes     = size_t(512) << 20; // of list items
+constexpr unsigned kMinItemCost = 1024;  // 16 evaluation batches
+constexpr unsigned kMaxItemCost = 16384;
+constexpr unsigned kHeavyCost   = 32768; // of the fused kernel's groups; compact ones cost about 17,000 at most
 
 /*! the groups of a traverse call are the caller's: each must hold 1 to 64 targets inside [firstBody, lastBody). A
  *  warp evaluates at most 64 targets, and an empty group would read before its start. The reference refuses
@@ -611,12 +591,65 @@ void checkCallerGroups(const ryo_group_view* grp, cudaStream_t stream)
                 "traverse: every group needs 1 to 64 targets within [firstBody, lastBody)");
 }
 
+/*! traverses t's groups, or those of @p list, through interaction lists until every group has been served or has
+ *  overflowed the stack. Lists are cut by the solve's group count and the walk alone, so a group's sums do not depend
+ *  on the launch or pass that it falls in. */
+void traverseLists(ryo_ctx* ctx, TraverseLaunch t, const uint32_t* list, uint32_t count, uint32_t solveGroups,
+                   bool ownStack, Control& c, cudaStream_t s)
+{
+    const uint32_t numGroups = uint32_t(t.numGroups);
+    // a caller's stack capacity is for one walk of the whole tree
+    t.subWalks  = (list || solveGroups <= kSubGroups) && ownStack ? 8 : 1;
+    t.itemCost  = std::min(kMaxItemCost, std::max(kMinItemCost, solveGroups / 2));
+    t.itemWords = t.subWalks > 1 ? 512 : 2048;
+    const size_t tasks = size_t(count) * t.subWalks;
+    // pieces per part of a walk seldom pass this; when they do, the groups that found no room walk again
+    const size_t pieces = (t.subWalks > 1 ? 6 : 3) * tasks;
+    t.itemCapacity      = uint32_t(std::min(pieces, kListBytes / (t.itemWords * sizeof(uint32_t))) + 4096);
+    t.taskLast          = ctx->scratch<int>("trav.taskLast", tasks, s);
+    t.groupState        = ctx->scratch<uint32_t>("trav.groupState", 3 * size_t(numGroups), s);
+    t.countM2P          = t.groupState + numGroups;
+    t.countP2P          = t.countM2P + numGroups;
+    RYO_CUDA(cudaMemsetAsync(t.groupState, 0, 3 * sizeof(uint32_t) * size_t(numGroups), s));
+    uint32_t* unserved[2] = {ctx->scratch<uint32_t>("trav.unservedA", count, s),
+                             ctx->scratch<uint32_t>("trav.unservedB", count, s)};
+    uint32_t chunk        = count; // groups per launch
+    for (int flip = 0;; flip ^= 1)
+    {
+        t.items      = ctx->scratch<ListItem>("trav.items", t.itemCapacity, s);
+        t.lists      = ctx->scratch<uint32_t>("trav.lists", size_t(t.itemCapacity) * t.itemWords, s);
+        t.partials   = ctx->scratch<float4>("trav.partials", size_t(t.itemCapacity) * 2 * kWarp, s);
+        uint32_t left = 0;
+        for (uint32_t first = 0; first < count; first += chunk)
+        {
+            t.groupList      = list ? list + first : nullptr;
+            t.numGroups      = int(std::min(chunk, count - first));
+            t.unservedGroups = unserved[flip] + left;
+            launchTraverse(t, ctx->smCount, s);
+            RYO_CUDA(cudaMemcpyAsync(&c, ctx->ctl, sizeof(Control), cudaMemcpyDeviceToHost, s));
+            RYO_CUDA(cudaStreamSynchronize(s));
+            left += c.unservedCount;
+            if (left > 0 || first + chunk < count) launchTraversalReset(ctx->ctl, kTravLists, s);
+        }
+        if (left == 0) return;
+        // groups that found no room walk again, fewer at a time; the pool grows only when it did not hold one group
+        if (chunk == 1) t.itemCapacity *= 4;
+        if (2 * left > count) chunk = std::max(1u, std::min(chunk, left) / 8);
+        list  = unserved[flip];
+        count = left;
+        launchResetGroups(list, count, t.groupState, t.countM2P, t.countP2P, s);
+    }
+}
+
+/*! run a traversal to completion: groups that overflow the stack are split in two along the SFC and traversed
+ *  again until none fails (traversal_gpu.cu:572-623); counts per group refer to the groups of @p t */
 void runTraversal(ryo_ctx* ctx, TraverseLaunch t, cudaStream_t s, double* potentialOut)
 {
     const uint32_t numGroups = uint32_t(t.numGroups);
     t.ctl                    = ctx->ctl;
-    if (t.stackCapacity <= 0) t.stackCapacity = 512; // the deepest walks measured use about 110 entries
-    launchTraversalReset(ctx->ctl, true, s);
+    const bool ownStack      = t.stackCapacity <= 0;
+    if (ownStack) t.stackCapacity = 512; // the deepest walks measured use about 110 entries
+    launchTraversalReset(ctx->ctl, kTravAll, s);
     ctx->retries          = 0;
     bool unsplittable     = false;
     uint32_t* failed      = ctx->scratch<uint32_t>("trav.failed", std::max<uint32_t>(numGroups, 1), s);
@@ -624,39 +657,30 @@ void runTraversal(ryo_ctx* ctx, TraverseLaunch t, cudaStream_t s, double* potent
     t.failedCapacity      = numGroups;
     int pass              = 0;
     bool flip             = false; // alternates the scratch buffers of successive split passes
-    // one threshold for every pass, from the solve's group count: a group's split decision depends on its cost and
-    // the solve's size, not on the launch or retry pass it falls in
-    const unsigned heavyCost = heavyCostFor(t.balanceGroups ? t.balanceGroups : numGroups, ctx->smCount);
+    const uint32_t solveGroups = t.balanceGroups ? t.balanceGroups : numGroups;
+    Control hc{};
     while (t.numGroups > 0)
     {
-        if (pass > 0) launchTraversalReset(ctx->ctl, false, s);
+        if (pass > 0) launchTraversalReset(ctx->ctl, kTravPass, s);
         ++pass;
-        // first pass: groups too costly for one warp are queued; second pass: each queued group split over warps
-        t.heavyGroups   = ctx->scratch<uint32_t>("trav.heavy", std::max(t.numGroups, 1), s);
-        t.heavyCapacity = uint32_t(t.numGroups);
-        t.heavyCost     = heavyCost;
-        t.parts         = 0;
-        t.numHeavy      = 0;
-        launchTraverse(t, ctx->smCount, s);
-        unsigned int counts[2] = {0, 0}; // failed, queued
-        RYO_CUDA(cudaMemcpyAsync(&counts[0], &ctx->ctl->failedCount, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
-        RYO_CUDA(cudaMemcpyAsync(&counts[1], &ctx->ctl->heavyCount, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
-        RYO_CUDA(cudaStreamSynchronize(s));
-        if (counts[1] > 0)
+        if (t.precision == kPrecisionF32 && solveGroups <= kListGroups)
+            traverseLists(ctx, t, nullptr, uint32_t(t.numGroups), solveGroups, ownStack, hc, s);
+        else
         {
-            TraverseLaunch t2 = t;
-            t2.numHeavy       = std::min(counts[1], t.heavyCapacity);
-            t2.parts          = heavyParts(t2.numHeavy, ctx->smCount);
-            size_t items      = size_t(t2.numHeavy) * size_t(t2.parts);
-            t2.partials       = ctx->scratch<float4>("trav.partials", items * 2 * kWarp, s);
-            t2.partStatus     = ctx->scratch<int>("trav.partStatus", items, s);
-            RYO_CUDA(cudaMemsetAsync(&ctx->ctl->workCounter, 0, sizeof(unsigned), s));
-            launchTraverse(t2, ctx->smCount, s);
-            launchCombineHeavy(t2, t.nodes ? t.tgtM : t.mt, s);
-            RYO_CUDA(cudaMemcpyAsync(&counts[0], &ctx->ctl->failedCount, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
+            t.heavyGroups   = ctx->scratch<uint32_t>("trav.heavy", std::max(t.numGroups, 1), s);
+            t.heavyCapacity = uint32_t(t.numGroups);
+            t.heavyCost     = kHeavyCost;
+            launchTraverse(t, ctx->smCount, s);
+            RYO_CUDA(cudaMemcpyAsync(&hc, ctx->ctl, sizeof(Control), cudaMemcpyDeviceToHost, s));
             RYO_CUDA(cudaStreamSynchronize(s));
+            if (hc.heavyCount > 0)
+            {
+                // groups too long for one warp go through lists, whose pieces all warps share
+                launchTraversalReset(ctx->ctl, kTravLists, s);
+                traverseLists(ctx, t, t.heavyGroups, hc.heavyCount, solveGroups, ownStack, hc, s);
+            }
         }
-        unsigned int numFailed = counts[0];
+        unsigned int numFailed = hc.failedCount;
         if (numFailed == 0) break;
         ctx->retries += numFailed;
         // split the failed groups on the device: halves along the SFC
@@ -696,9 +720,6 @@ void runTraversal(ryo_ctx* ctx, TraverseLaunch t, cudaStream_t s, double* potent
         t.failedGroups   = failed;
         t.failedCapacity = uint32_t(t.numGroups);
     }
-    Control hc;
-    RYO_CUDA(cudaMemcpyAsync(&hc, ctx->ctl, sizeof(Control), cudaMemcpyDeviceToHost, s));
-    RYO_CUDA(cudaStreamSynchronize(s));
     for (int i = 0; i < 5; ++i)
         ctx->hostStats[i] = hc.stats[i];
     if (unsplittable) ctx->hostStats[kMaxP2P] = 0xFFFFFFFFull;

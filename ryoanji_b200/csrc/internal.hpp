@@ -25,7 +25,10 @@ struct Control
     double potential;          // sum m * phi of the traversal (no G)
     double ewaldPotential;     // sum m * phi of the Ewald correction (no G)
     unsigned int counters[8];  // scratch counters for other kernels
-    unsigned int heavyCount;   // groups queued for the split second traversal pass
+    unsigned int heavyCount;   // groups queued for the interaction-list kernels
+    unsigned int itemCount;    // items of the interaction lists, and the head of their queue
+    unsigned int itemHead;
+    unsigned int unservedCount; // groups whose list did not fit into the pool
 };
 
 enum BhStat
@@ -302,6 +305,19 @@ void launchPackBodies(const float* x, const float* y, const float* z, const floa
                       cudaStream_t s);
 
 // ---------------------------------------------------------------------------------------------------- traverse.cu
+//! a piece of a group's interaction list
+struct alignas(16) ListItem
+{
+    uint32_t group; // target group
+    uint32_t words; // words used
+    int prev;       // the item before it in the walk, -1 for the first
+    uint32_t only;  // 1 if it is the group's only item
+};
+
+//! why a group was not evaluated: its walk overflowed the stack, or found no free slot
+constexpr uint32_t kGroupFailed   = 1;
+constexpr uint32_t kGroupUnserved = 2;
+
 struct TraverseLaunch
 {
     const uint32_t* groupStart;
@@ -344,19 +360,27 @@ struct TraverseLaunch
     const uint32_t* groupSys;
     const struct SysTrav* systems;
     double* sysPotential;
-    // groups too costly for one warp. First pass (parts == 0, heavyGroups set): a group whose interaction count
-    // (direct bodies + 2 x approximated cells) passes heavyCost stops and is queued in heavyGroups. Second pass
-    // (parts > 0): item i walks group heavyGroups[i / parts] in full but evaluates only every parts-th batch,
-    // starting at batch i % parts, and writes its compensated partial sums to partials[i][64] for the combine step.
-    uint32_t balanceGroups; // group count the split threshold follows (0: the launch's); a solve traversed in several
-                            // launches passes its total, so that its groups split as in one launch
+    uint32_t balanceGroups; // group count that decides how lists are used and cut (0: the launch's); a solve traversed
+                            // in several launches passes its total, so that its groups sum as in one launch
+    // subWalks 0: the fused kernel; a group whose interaction count (direct bodies + 2 x approximated cells) passes
+    // heavyCost stops and is queued in heavyGroups
     uint32_t* heavyGroups;
     uint32_t heavyCapacity;
     unsigned heavyCost;
-    int parts;
-    uint32_t numHeavy;  // second pass: queued groups
-    float4* partials;   // second pass: (-phi, ax, ay, az) of the group's 64 targets, per item
-    int* partStatus;    // second pass: per item, 1 if the walk overflowed the stack
+    // else the interaction-list kernels, for all groups or those in groupList: walks in subWalks parts (1, or 8) write
+    // items of itemWords words, closed past itemCost interactions
+    uint32_t subWalks;
+    const uint32_t* groupList;
+    ListItem* items;
+    uint32_t* lists;
+    float4* partials;       // (-phi, ax, ay, az) of an item's 64 targets
+    uint32_t itemCapacity, itemWords;
+    unsigned itemCost;
+    int* taskLast;          // per part of a walk: its last item, -1 if its list is empty
+    uint32_t* groupState;   // per group: 0, kGroupFailed or kGroupUnserved
+    uint32_t* countM2P;     // per group, of the walk
+    uint32_t* countP2P;
+    uint32_t* unservedGroups;
     // min and max softening of every target and source as ordered bits (null: not known). Equal values let the
     // direct sums skip staging and comparing the sources' softening.
     const uint32_t* softeningRange;
@@ -398,10 +422,11 @@ struct SysTrav
 void launchBatchSofteningRange(const float* h, const float* m, const uint64_t* first, uint32_t numSystems,
                                SysTrav* trav, cudaStream_t s);
 void launchTraverse(const TraverseLaunch& t, int smCount, cudaStream_t s);
-/*! after a second pass: per queued group, the parts' partial sums added in part order into the outputs (and the
- *  potential); a group whose walk overflowed the stack goes to t.failedGroups instead. @p mass: target masses */
-void launchCombineHeavy(const TraverseLaunch& t, const float* mass, cudaStream_t s);
-void launchTraversalReset(Control* ctl, bool resetStats, cudaStream_t s);
+//! what a reset clears: the statistics and all counters, a pass's counters, or those of the interaction lists
+constexpr int kTravAll = 0, kTravPass = 1, kTravLists = 2;
+void launchTraversalReset(Control* ctl, int what, cudaStream_t s);
+void launchResetGroups(const uint32_t* list, uint32_t n, uint32_t* state, uint32_t* m2p, uint32_t* p2p,
+                       cudaStream_t s);
 
 // ---------------------------------------------------------------------------------------------------- groups.cu
 //! the reference's default window-extent ratio (8, or CSTONE_GROUP_EXTENT_SPLIT)

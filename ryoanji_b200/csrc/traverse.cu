@@ -9,6 +9,14 @@
  *
  * B200 design:
  *   - persistent warps pull 64-body target groups from a per-context work counter; each lane owns two targets;
+ *   - two forms. The fused kernel walks and evaluates a group in one warp. It is bound by the FP32 pipe, and takes
+ *     launches of many groups, which balance by themselves. Launches of few groups, and groups far too long for one
+ *     warp, go through interaction lists: walkKernel writes each group's cells and direct leaves to pieces of bounded
+ *     cost, evalKernel evaluates the pieces in any order, finishKernel adds them up. A solve's time is then no longer
+ *     that of its longest group. Traversal of a Plummer sphere of 60,001 bodies (938 groups, the longest seven times
+ *     the mean): 0.48 ms, against 1.24 ms by the fused kernel with its longest groups repeated by several warps; of
+ *     2^20 bodies: 6.8 against 7.4 ms; of 256 batched spheres (42,002 groups): 8.2 against 8.9 ms. From about 50,000
+ *     groups the fused kernel is as fast and needs no lists;
  *   - depth-first traversal over a per-warp stack in shared memory (entries are the first of eight siblings;
  *     four entries, 32 cells, are tested per step), bounded by the stack capacity; a group that would exceed it is
  *     reported and split by the host, as the reference does with its global queue;
@@ -35,12 +43,27 @@ constexpr int kTravThreads  = kTravWarps * kWarp;
 constexpr int kM2PCap       = 64;  // pending approximated cells (flushed at 64, or 32 for dipole expansions)
 constexpr int kLeafCap      = 64;  // pending direct leaves (flushed when more than 32 are pending)
 constexpr int kP2PBatch     = 2 * kWarp; // direct bodies evaluated per staging round (two per lane)
+constexpr int kEvalBlocks   = 5;     // resident blocks of the list evaluation per SM (4: 1-2% slower, 6: 2-3%)
+constexpr int kSegLeafCap   = kWarp; // direct leaves per list segment
 constexpr int kRootOnly     = -2;  // stack marker: the root itself is the only cell (single-leaf tree); a marker
                                    // -(r + 2) stands for the single cell r
+
+// segment header of an interaction list: kind in the low two bits, entry count above
+constexpr uint32_t kSegCells = 0, kSegLeaves = 1, kSegReplica = 2, kSegImages = 3;
+constexpr int kReplicaWords  = 4;
+
+//! a list walk's pending entries: a segment leaves fewer than a segment's, and one walk step adds at most kWarp
+struct WalkSmem
+{
+    int m2p[kM2PCap + kWarp];
+    uint32_t image[kM2PCap + kWarp]; // of periodic groups: the image each pending cell is seen in
+    int2 leaves[kSegLeafCap + kWarp];
+};
 
 struct WarpSmem
 {
     int m2p[kM2PCap + kWarp];
+    uint32_t image[kM2PCap]; // lists of periodic groups: the image each pending cell is seen in
     int2 leaves[kLeafCap + kWarp];
     int leafScan[kLeafCap + kWarp];
     // staged sources, every value duplicated: M2P 5 x 16 bytes per cell for 64 quadrupoles (7 for 32 dipole
@@ -48,9 +71,6 @@ struct WarpSmem
     float4 stage[10 * kWarp];
     // per lane: Kahan running sums [0] and compensations [1] of (-phi, ax, ay, az), both targets packed
     unsigned long long sums[2][4][kWarp];
-    // evaluation batches of the current walk: the next batch's number, and which of them this warp evaluates
-    // (batch j when j % parts == part; parts is 1 outside the split second pass)
-    int batchNext, part, parts, item;
     // 1 if every target and source of the launch has the softening of the group's targets (T.h0)
     int allUniform;
     // 1 if every source of the launch has the mass massU: the direct sums then apply it once per batch
@@ -59,21 +79,8 @@ struct WarpSmem
     int pad;
 };
 
-//! true if the walk's next evaluation batch belongs to this warp; counts the batch either way. Outside the split
-//! second pass (kSplit false) every batch is the warp's own.
-template<bool kSplit>
-__device__ __forceinline__ bool ownBatch(WarpSmem& S)
-{
-    if constexpr (!kSplit) return true;
-    int j = S.batchNext;
-    __syncwarp();
-    if (laneId() == 0) S.batchNext = j + 1;
-    __syncwarp();
-    return S.parts <= 1 || j % S.parts == S.part;
-}
-
 static_assert(2 * kP2PBatch + kP2PBatch / 2 <= 10 * kWarp, "a P2P batch must fit in the stage");
-static_assert(5 * 2 * kWarp <= 10 * kWarp && 7 * kWarp <= 10 * kWarp, "an M2P batch must fit in the stage");
+static_assert(5 * 2 * kWarp <= 10 * kWarp && 9 * kWarp <= 10 * kWarp, "an M2P batch must fit in the stage");
 // an M2P flush leaves fewer than kWarp cells pending (at most 64 + 31 before it); one walk step adds at most kWarp
 static_assert(2 * kWarp - 1 + kWarp <= kM2PCap + kWarp, "the pending cell list must hold a step's additions");
 // a P2P evaluation leaves fewer than kP2PBatch bodies, so at most kP2PBatch - 1 leaves, pending; one walk step adds
@@ -244,6 +251,14 @@ struct TargetState
     f2 tx, ty, tz, th; // the lane's two targets (shifted by the current replica)
     float h0;          // the common smoothing length of the group's targets, if uniformH
     bool uniformH;
+
+    __device__ __forceinline__ void set(const float4& t0, const float4& t1)
+    {
+        tx = pk(t0.x, t1.x);
+        ty = pk(t0.y, t1.y);
+        tz = pk(t0.z, t1.z);
+        th = pk(t0.w, t1.w);
+    }
 };
 
 __device__ __forceinline__ void kahan2(f2& sum, f2& comp, f2 v)
@@ -382,20 +397,35 @@ __device__ __forceinline__ void addBatchS(WarpSmem& S, const Acc2& part)
     }
 }
 
-//! approximated cells per evaluation batch: 64 quadrupoles (5 staged float4 each), or 32 dipole expansions (7)
-template<class Nodes>
-__host__ __device__ constexpr int m2pBatch()
+//! a periodic image (ix, iy, iz), each in [-kMaxImage, kMaxImage), in one word, and its components
+constexpr int kMaxImage = 512;
+__device__ __forceinline__ uint32_t packImage(int ix, int iy, int iz)
 {
-    return Nodes::kDipole ? kWarp : 2 * kWarp;
+    return uint32_t(ix + kMaxImage) | (uint32_t(iy + kMaxImage) << 10) | (uint32_t(iz + kMaxImage) << 20);
+}
+__device__ __forceinline__ float imageShift(uint32_t image, int d)
+{
+    return float(int((image >> (10 * d)) & 1023u) - kMaxImage);
 }
 
-//! evaluate the first @p count (<= m2pBatch) pending cells
-template<bool kSplit, class Nodes>
-__device__ void evalM2P(WarpSmem& S, int count, const Nodes& nodes, TargetState& T)
+//! approximated cells per evaluation batch: 64 quadrupoles (5 staged float4 each), or 32 dipole expansions (7) or
+//! cells with a shift (7, or 9 with a dipole)
+template<class Nodes, bool kImages = false>
+__host__ __device__ constexpr int m2pBatch()
 {
-    constexpr int kStride = Nodes::kDipole ? 7 : 5; // staged float4 per cell
-    constexpr int kBatch  = m2pBatch<Nodes>();
-    if (!ownBatch<kSplit>(S)) return;
+    return Nodes::kDipole || kImages ? kWarp : 2 * kWarp;
+}
+
+/*! evaluate @p count (<= m2pBatch) pending cells from the @p first on. With kImages the cells belong to several replicas
+ *  of a periodic box and every cell's shift is staged too: a pair's distance is (target + shift) - cell, as where the
+ *  targets are moved. */
+template<bool kImages = false, class Nodes>
+__device__ __forceinline__ void evalM2P(WarpSmem& S, int first, int count, const Nodes& nodes, const TargetState& T,
+                                        const float* boxL = nullptr)
+{
+    constexpr int kCell   = Nodes::kDipole ? 7 : 5;
+    constexpr int kStride = kCell + (kImages ? 2 : 0); // staged float4 per cell
+    constexpr int kBatch  = m2pBatch<Nodes, kImages>();
     int lane = laneId();
 #pragma unroll
     for (int half = 0; half < kBatch / kWarp; ++half)
@@ -404,7 +434,7 @@ __device__ void evalM2P(WarpSmem& S, int count, const Nodes& nodes, TargetState&
         if (k < count)
         {
             float4 c, q0, q1, dp = make_float4(0.f, 0.f, 0.f, 0.f);
-            nodes.multipole(S.m2p[k], c, q0, q1, dp);
+            nodes.multipole(S.m2p[first + k], c, q0, q1, dp);
             float4* st = S.stage + kStride * k;
             st[0]      = make_float4(c.x, c.x, c.y, c.y);
             st[1]      = make_float4(c.z, c.z, q0.x, q0.x);
@@ -416,6 +446,14 @@ __device__ void evalM2P(WarpSmem& S, int count, const Nodes& nodes, TargetState&
                 st[5 % kStride] = make_float4(dp.x, dp.x, dp.y, dp.y);
                 st[6 % kStride] = make_float4(dp.z, dp.z, 0.f, 0.f);
             }
+            if constexpr (kImages)
+            {
+                const uint32_t im = S.image[first + k];
+                const float sx = __fmul_rn(imageShift(im, 0), boxL[0]), sy = __fmul_rn(imageShift(im, 1), boxL[1]),
+                            sz = __fmul_rn(imageShift(im, 2), boxL[2]);
+                st[kCell]      = make_float4(sx, sx, sy, sy);
+                st[kCell + 1]  = make_float4(sz, sz, 0.f, 0.f);
+            }
         }
     }
     __syncwarp();
@@ -425,13 +463,19 @@ __device__ void evalM2P(WarpSmem& S, int count, const Nodes& nodes, TargetState&
     {
         const ulonglong2* sj = st + kStride * j;
         ulonglong2 a = sj[0], b = sj[1], c = sj[2], d = sj[3], e = sj[4];
+        f2 tx = T.tx, ty = T.ty, tz = T.tz;
+        if constexpr (kImages)
+        {
+            ulonglong2 u = sj[kCell], v = sj[kCell + 1];
+            tx = add2(tx, u.x), ty = add2(ty, u.y), tz = add2(tz, v.x);
+        }
         if constexpr (Nodes::kDipole)
         {
             ulonglong2 f = sj[5 % kStride], g = sj[6 % kStride];
-            m2p2mdq(part, T.tx, T.ty, T.tz, a.x, a.y, b.x, b.y, c.x, c.y, d.x, d.y, e.x, e.y, f.x, f.y, g.x);
+            m2p2mdq(part, tx, ty, tz, a.x, a.y, b.x, b.y, c.x, c.y, d.x, d.y, e.x, e.y, f.x, f.y, g.x);
         }
         else
-            m2p2(part, T.tx, T.ty, T.tz, a.x, a.y, b.x, b.y, c.x, c.y, d.x, d.y, e.x, e.y);
+            m2p2(part, tx, ty, tz, a.x, a.y, b.x, b.y, c.x, c.y, d.x, d.y, e.x, e.y);
     };
     if (count == kBatch)
     {
@@ -458,8 +502,8 @@ __device__ void evalM2P(WarpSmem& S, int count, const Nodes& nodes, TargetState&
 
 /*! evaluate pending direct leaves in batches of kP2PBatch bodies; with @p all == false only whole batches are evaluated
  *  and the remainder stays pending (the first pending leaf may be partly consumed). Returns the leaves left. */
-template<bool kSplit, class Sources>
-__device__ int evalP2P(WarpSmem& S, int numLeaves, bool all, const Sources& src, TargetState& T)
+template<class Sources>
+__device__ __forceinline__ int evalP2P(WarpSmem& S, int numLeaves, bool all, const Sources& src, const TargetState& T)
 {
     int lane = laneId();
     // inclusive scan of the body counts over the pending leaves
@@ -493,7 +537,6 @@ __device__ int evalP2P(WarpSmem& S, int numLeaves, bool all, const Sources& src,
         const unsigned long long ends = (static_cast<unsigned long long>(endsHi) << 32) | endsLo;
         const int leafBase = first;
         first += __popcll(ends); // the leaves ending inside this batch come before the next batch's first body
-        if (!ownBatch<kSplit>(S)) continue;
 #pragma unroll
         for (int half = 0; half < 2; ++half)
         {
@@ -648,25 +691,44 @@ __device__ int evalP2P(WarpSmem& S, int numLeaves, bool all, const Sources& src,
     return keep;
 }
 
-__global__ void resetTraversal(Control* ctl, bool resetStats)
+//! statistics and counters at the start of a traversal, a pass's counters, or those of its interaction lists
+__global__ void resetTraversal(Control* ctl, int what)
 {
-    if (threadIdx.x == 0)
+    if (threadIdx.x != 0) return;
+    ctl->workCounter   = 0;
+    ctl->itemCount     = 0;
+    ctl->itemHead      = 0;
+    ctl->unservedCount = 0;
+    if (what == kTravLists) return;
+    ctl->failedCount = 0;
+    ctl->heavyCount  = 0;
+    if (what == kTravAll)
     {
-        ctl->workCounter = 0;
-        ctl->failedCount = 0;
-        ctl->heavyCount  = 0;
-        if (resetStats)
-        {
-            for (int i = 0; i < 5; ++i)
-                ctl->stats[i] = 0;
-            ctl->potential = 0.0;
-        }
+        for (int i = 0; i < 5; ++i)
+            ctl->stats[i] = 0;
+        ctl->potential = 0.0;
     }
 }
 
-void launchTraversalReset(Control* ctl, bool resetStats, cudaStream_t s)
+void launchTraversalReset(Control* ctl, int what, cudaStream_t s)
 {
-    resetTraversal<<<1, 32, 0, s>>>(ctl, resetStats);
+    resetTraversal<<<1, 32, 0, s>>>(ctl, what);
+    RYO_LAUNCH_CHECK();
+}
+
+//! makes the groups of a list ready to be walked again
+__global__ void resetGroups(const uint32_t* __restrict__ list, uint32_t n, uint32_t* state, uint32_t* m2p,
+                            uint32_t* p2p)
+{
+    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    uint32_t g = list[i];
+    state[g] = m2p[g] = p2p[g] = 0;
+}
+
+void launchResetGroups(const uint32_t* list, uint32_t n, uint32_t* state, uint32_t* m2p, uint32_t* p2p, cudaStream_t s)
+{
+    resetGroups<<<ceilDiv(n, 256), 256, 0, s>>>(list, n, state, m2p, p2p);
     RYO_LAUNCH_CHECK();
 }
 
@@ -681,66 +743,107 @@ __device__ __forceinline__ void storeResult(const TraverseLaunch& P, int idx, fl
     P.az[idx] = (add ? P.az[idx] : 0.f) + z;
 }
 
-//! one warp per queued group: add the parts' partial sums in part order (FP64) and write the group's results
-__global__ void combineHeavyKernel(TraverseLaunch P, const float* __restrict__ mass)
+//! the tree root and periodic images of a group: the launch's, or its system's in a batched solve
+struct GroupFrame
 {
-    const unsigned w    = (blockIdx.x * blockDim.x + threadIdx.x) / kWarp;
-    const unsigned lane = laneId();
-    if (w >= P.numHeavy) return; // whole warps leave together
-    const unsigned g   = P.heavyGroups[w];
-    const int K        = P.parts;
-    const size_t item0 = size_t(w) * unsigned(K);
-    bool failed        = false;
-    for (int k = int(lane); k < K; k += kWarp)
-        failed |= P.partStatus[item0 + k] != 0;
-    if (__any_sync(0xffffffffu, failed))
+    int rootEntry, shells;
+    float boxL[3];
+    uint32_t sys;
+
+    __device__ __forceinline__ void set(const TraverseLaunch& P, unsigned g)
     {
-        if (lane == 0)
+        rootEntry = P.numNodes == 1 ? kRootOnly : P.initNode;
+        shells    = P.numShells;
+        sys       = 0;
+        if (P.groupSys)
         {
-            unsigned slotF = atomicAdd(&P.ctl->failedCount, 1u);
-            if (slotF < P.failedCapacity) P.failedGroups[slotF] = g;
-        }
-        return;
-    }
-    const int b = int(P.groupStart[g]), e = int(P.groupEnd[g]);
-    double pot  = 0.0;
+            sys               = P.groupSys[g];
+            const SysTrav& st = P.systems[sys];
+            rootEntry         = st.entry;
+            shells            = st.numShells;
 #pragma unroll
-    for (int t = 0; t < 2; ++t)
-    {
-        double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
-        for (int k = 0; k < K; ++k)
-        {
-            float4 v = P.partials[(item0 + k) * (2 * kWarp) + t * kWarp + lane];
-            s0 += v.x;
-            s1 += v.y;
-            s2 += v.z;
-            s3 += v.w;
+            for (int d = 0; d < 3; ++d)
+                boxL[d] = st.boxL[d];
         }
-        int idx = b + t * kWarp + int(lane);
+        else
+        {
+#pragma unroll
+            for (int d = 0; d < 3; ++d)
+                boxL[d] = P.boxL[d];
+        }
+    }
+};
+
+//! whether the targets' softening, and the sources' mass, are one for all bodies: those of the launch, or in a batched
+//! solve the system's, whose groups meet only its own bodies
+__device__ __forceinline__ void setUniform(const TraverseLaunch& P, const GroupFrame& F, const TargetState& T,
+                                           WarpSmem& S)
+{
+    if (laneId() != 0) return;
+    const bool knownH = P.groupSys || P.softeningRange;
+    const bool knownM = P.groupSys || P.massRange;
+    uint32_t hLo = 0, hHi = 1, mLo = 0, mHi = 1;
+    if (P.groupSys)
+    {
+        const SysTrav& st = P.systems[F.sys];
+        hLo = st.hLo, hHi = st.hHi, mLo = st.mLo, mHi = st.mHi;
+    }
+    else
+    {
+        if (knownH) hLo = P.softeningRange[0], hHi = P.softeningRange[1];
+        if (knownM) mLo = P.massRange[0], mHi = P.massRange[1];
+    }
+    S.allUniform  = knownH && T.uniformH && hLo == hHi && orderedFloat(hLo) == T.h0;
+    S.uniformMass = knownM && mLo == mHi;
+    S.massU       = S.uniformMass ? orderedFloat(mLo) : 0.f;
+}
+
+//! phi and acceleration sums of a lane's two targets
+struct ListSums
+{
+    float phi[2], x[2], y[2], z[2];
+};
+
+//! Kahan: the compensated sum is sums - compensation; sums[.][0] holds -phi
+__device__ __forceinline__ ListSums readSums(const WarpSmem& S)
+{
+    const int lane = laneId();
+    ListSums r;
+    upk(sub2(S.sums[1][0][lane], S.sums[0][0][lane]), r.phi[0], r.phi[1]);
+    upk(sub2(S.sums[0][1][lane], S.sums[1][1][lane]), r.x[0], r.x[1]);
+    upk(sub2(S.sums[0][2][lane], S.sums[1][2][lane]), r.y[0], r.y[1]);
+    upk(sub2(S.sums[0][3][lane], S.sums[1][3][lane]), r.z[0], r.z[1]);
+    return r;
+}
+
+//! the results of the group [b, e) of system @p sys
+template<class Targets>
+__device__ __forceinline__ void storeGroup(const TraverseLaunch& P, const Targets& tgt, const ListSums& r, int b, int e,
+                                           uint32_t sys)
+{
+    double pot = 0.0;
+#pragma unroll
+    for (int k = 0; k < 2; ++k)
+    {
+        int idx = b + k * kWarp + int(laneId());
         if (idx < e)
         {
-            float phi = float(s0), gx = float(s1), gy = float(s2), gz = float(s3);
-            float mi  = mass[idx];
-            pot += double(mi) * double(phi);
-            storeResult(P, idx, P.G * mi * phi, P.G * gx, P.G * gy, P.G * gz);
+            float mi = tgt.scalar(idx);
+            pot += double(mi) * double(r.phi[k]);
+            storeResult(P, idx, P.G * mi * r.phi[k], P.G * r.x[k], P.G * r.y[k], P.G * r.z[k]);
         }
     }
     pot = warpSum(pot);
-    if (lane == 0)
+    if (laneId() == 0)
     {
         atomicAdd(&P.ctl->potential, pot);
-        if (P.sysPotential) atomicAdd(P.sysPotential + (P.groupSys ? P.groupSys[g] : 0u), pot);
+        if (P.sysPotential) atomicAdd(P.sysPotential + sys, pot);
     }
 }
 
-void launchCombineHeavy(const TraverseLaunch& t, const float* mass, cudaStream_t s)
-{
-    if (t.numHeavy == 0) return;
-    combineHeavyKernel<<<ceilDiv(size_t(t.numHeavy) * kWarp, 256), 256, 0, s>>>(t, mass);
-    RYO_LAUNCH_CHECK();
-}
-
-template<class Nodes, class Targets, class Sources, bool kSplit>
+/*! the traversal of a launch of many groups: a warp walks the tree for a group and evaluates its batches on the way. A
+ *  group whose interaction count passes P.heavyCost stops and is queued for the interaction-list kernels below. */
+template<class Nodes, class Targets, class Sources>
 __global__ void __launch_bounds__(kTravThreads, 5)
     traverseKernel(TraverseLaunch P, Nodes nodes, Targets tgt, Sources src)
 {
@@ -750,40 +853,20 @@ __global__ void __launch_bounds__(kTravThreads, 5)
     WarpSmem& S    = reinterpret_cast<WarpSmem*>(smemRaw + sizeof(int) * kTravWarps * P.stackCapacity)[warp];
     const unsigned lt = lanemaskLt();
 
-    const unsigned numItems = P.parts > 0 ? P.numHeavy * unsigned(P.parts) : unsigned(P.numGroups);
     while (true)
     {
-        unsigned item = 0;
-        if (lane == 0) item = atomicAdd(&P.ctl->workCounter, 1u);
-        item = __shfl_sync(0xffffffffu, item, 0);
-        if (item >= numItems) return;
-        unsigned g = item;
-        if (P.parts > 0) g = P.heavyGroups[item / unsigned(P.parts)];
-        if (lane == 0)
-        {
-            S.batchNext = 0;
-            S.part      = P.parts > 0 ? int(item % unsigned(P.parts)) : 0;
-            S.parts     = P.parts > 0 ? P.parts : 1;
-            S.item      = int(item);
-        }
+        unsigned g = 0;
+        if (lane == 0) g = atomicAdd(&P.ctl->workCounter, 1u);
+        g = __shfl_sync(0xffffffffu, g, 0);
+        if (g >= unsigned(P.numGroups)) return;
 
         const int b = int(P.groupStart[g]), e = int(P.groupEnd[g]);
         TargetState T;
         float4 t0 = tgt.vec(min(b + lane, e - 1));
         float4 t1 = tgt.vec(min(b + kWarp + lane, e - 1));
-        T.tx      = pk(t0.x, t1.x);
-        T.ty      = pk(t0.y, t1.y);
-        T.tz      = pk(t0.z, t1.z);
-        T.th      = pk(t0.w, t1.w);
+        T.set(t0, t1);
         T.h0       = __shfl_sync(0xffffffffu, t0.w, 0);
         T.uniformH = __all_sync(0xffffffffu, t0.w == T.h0 && t1.w == T.h0);
-        if (lane == 0)
-        {
-            S.allUniform = P.softeningRange && T.uniformH && P.softeningRange[0] == P.softeningRange[1] &&
-                           orderedFloat(P.softeningRange[0]) == T.h0;
-            S.uniformMass = P.massRange && !P.groupSys && P.massRange[0] == P.massRange[1];
-            S.massU       = S.uniformMass ? orderedFloat(P.massRange[0]) : 0.f;
-        }
 #pragma unroll
         for (int c = 0; c < 4; ++c)
             S.sums[0][c][lane] = S.sums[1][c][lane] = 0ull;
@@ -798,33 +881,14 @@ __global__ void __launch_bounds__(kTravThreads, 5)
             ts[d]   = __fmul_rn(__fsub_rn(h, l), 0.5f);
         }
 
-        // the group's tree root and periodic images: the launch's, or its system's in a batched solve
-        int rootEntry = P.numNodes == 1 ? kRootOnly : P.initNode;
-        int shells    = P.numShells;
-        float boxL[3] = {P.boxL[0], P.boxL[1], P.boxL[2]};
-        uint32_t sys  = 0;
-        if (P.groupSys)
-        {
-            sys               = P.groupSys[g];
-            const SysTrav& st = P.systems[sys];
-            rootEntry         = st.entry;
-            // a system's groups meet only its own bodies: its own softening range decides
-            if (lane == 0)
-            {
-                S.allUniform  = T.uniformH && st.hLo == st.hHi && orderedFloat(st.hLo) == T.h0;
-                S.uniformMass = st.mLo == st.mHi;
-                S.massU       = S.uniformMass ? orderedFloat(st.mLo) : 0.f;
-            }
-            shells            = st.numShells;
-            boxL[0]           = st.boxL[0];
-            boxL[1]           = st.boxL[1];
-            boxL[2]           = st.boxL[2];
-        }
+        GroupFrame F;
+        F.set(P, g);
+        setUniform(P, F, T, S);
 
         unsigned nM2P = 0, nP2P = 0;
         int maxStack  = 0;
         bool overflow = false, heavy = false;
-        const bool mayQueue = P.parts == 0 && P.heavyGroups != nullptr;
+        const int shells = F.shells;
         for (int iz = -shells; iz <= shells && !overflow; ++iz)
             for (int iy = -shells; iy <= shells && !overflow; ++iy)
                 for (int ix = -shells; ix <= shells && !overflow; ++ix)
@@ -834,8 +898,8 @@ __global__ void __launch_bounds__(kTravThreads, 5)
                     // are the original positions plus the shift: shifting them back and forth as the reference
                     // does leaves rounding residues, and a target then meets itself at about one float ulp of the
                     // box coordinates, which a softening below that turns into a large spurious force.
-                    float sh[3] = {__fmul_rn(float(ix), boxL[0]), __fmul_rn(float(iy), boxL[1]),
-                                   __fmul_rn(float(iz), boxL[2])};
+                    float sh[3] = {__fmul_rn(float(ix), F.boxL[0]), __fmul_rn(float(iy), F.boxL[1]),
+                                   __fmul_rn(float(iz), F.boxL[2])};
 #pragma unroll
                     for (int d = 0; d < 3; ++d)
                         tc[d] = __fadd_rn(tc[d], sh[d]);
@@ -849,7 +913,7 @@ __global__ void __launch_bounds__(kTravThreads, 5)
                     }
 
                     int sp = 1, nM = 0, nL = 0;
-                    if (lane == 0) stack[0] = rootEntry;
+                    if (lane == 0) stack[0] = F.rootEntry;
                     __syncwarp();
                     while (sp > 0)
                     {
@@ -896,9 +960,9 @@ __global__ void __launch_bounds__(kTravThreads, 5)
                         nL += __popc(bl);
                         nP2P += __reduce_add_sync(0xffffffffu, hasB ? unsigned(link.z) : 0u);
                         __syncwarp();
-                        if (mayQueue && nP2P + 2u * nM2P > P.heavyCost)
+                        if (nP2P + 2u * nM2P > P.heavyCost)
                         {
-                            // too much for one warp: leave it to the split second pass
+                            // too much for one warp: leave it to the list kernels
                             heavy    = true;
                             overflow = true;
                             break;
@@ -907,17 +971,17 @@ __global__ void __launch_bounds__(kTravThreads, 5)
                         constexpr int kMB = m2pBatch<Nodes>();
                         while (nM >= kMB)
                         {
-                            evalM2P<kSplit>(S, kMB, nodes, T);
+                            evalM2P(S, 0, kMB, nodes, T);
                             nM -= kMB; // fewer than kWarp cells remain: one move per lane
                             if (lane < nM) S.m2p[lane] = S.m2p[kMB + lane];
                             __syncwarp();
                         }
-                        if (nL > kLeafCap - kWarp) nL = evalP2P<kSplit>(S, nL, false, src, T);
+                        if (nL > kLeafCap - kWarp) nL = evalP2P(S, nL, false, src, T);
                     }
                     if (!overflow)
                     {
-                        if (nM > 0) evalM2P<kSplit>(S, nM, nodes, T);
-                        if (nL > 0) evalP2P<kSplit>(S, nL, true, src, T);
+                        if (nM > 0) evalM2P(S, 0, nM, nodes, T);
+                        if (nL > 0) evalP2P(S, nL, true, src, T);
                     }
 #pragma unroll
                     for (int d = 0; d < 3; ++d)
@@ -935,57 +999,17 @@ __global__ void __launch_bounds__(kTravThreads, 5)
         }
         if (overflow)
         {
-            // write nothing; the host splits the group and traverses the halves again (in the second pass the
-            // combine step reports the group)
-            if (P.parts > 0)
-            {
-                if (lane == 0) P.partStatus[S.item] = 1;
-                if (S.part != 0) continue;
-            }
+            // write nothing; the host splits the group and traverses the halves again
             if (lane == 0)
             {
-                if (P.parts == 0)
-                {
-                    unsigned slotF = atomicAdd(&P.ctl->failedCount, 1u);
-                    if (slotF < P.failedCapacity) P.failedGroups[slotF] = g;
-                }
+                unsigned slotF = atomicAdd(&P.ctl->failedCount, 1u);
+                if (slotF < P.failedCapacity) P.failedGroups[slotF] = g;
                 atomicMax(&P.ctl->stats[kMaxStack], (unsigned long long)maxStack);
             }
             continue;
         }
 
-        // Kahan: the compensated sum is acc - comp; acc.p holds -phi
-        float phi[2], gx[2], gy[2], gz[2];
-        upk(sub2(S.sums[1][0][lane], S.sums[0][0][lane]), phi[0], phi[1]);
-        upk(sub2(S.sums[0][1][lane], S.sums[1][1][lane]), gx[0], gx[1]);
-        upk(sub2(S.sums[0][2][lane], S.sums[1][2][lane]), gy[0], gy[1]);
-        upk(sub2(S.sums[0][3][lane], S.sums[1][3][lane]), gz[0], gz[1]);
-        double pot = 0.0;
-        if (P.parts > 0)
-        {
-            // this part's share; the combine step adds the parts in order. Every part walked the whole group, so
-            // part 0 reports the group's interaction counts.
-            float4* out       = P.partials + size_t(S.item) * (2 * kWarp);
-            out[lane]         = make_float4(phi[0], gx[0], gy[0], gz[0]);
-            out[kWarp + lane] = make_float4(phi[1], gx[1], gy[1], gz[1]);
-            if (lane == 0) P.partStatus[S.item] = 0;
-            if (S.part != 0) continue;
-        }
-        else
-        {
-#pragma unroll
-            for (int k = 0; k < 2; ++k)
-            {
-                int idx = b + k * kWarp + lane;
-                if (idx < e)
-                {
-                    float mi = tgt.scalar(idx);
-                    pot += double(mi) * double(phi[k]);
-                    storeResult(P, idx, P.G * mi * phi[k], P.G * gx[k], P.G * gy[k], P.G * gz[k]);
-                }
-            }
-            pot = warpSum(pot);
-        }
+        storeGroup(P, tgt, readSums(S), b, e, P.groupSys ? P.groupSys[g] : 0u);
         if (lane == 0)
         {
             unsigned long long size = (unsigned long long)(e - b);
@@ -994,38 +1018,557 @@ __global__ void __launch_bounds__(kTravThreads, 5)
             atomicMax(&P.ctl->stats[kMaxM2P], (unsigned long long)nM2P);
             atomicAdd(&P.ctl->stats[kSumM2P], (unsigned long long)nM2P * size);
             atomicMax(&P.ctl->stats[kMaxStack], (unsigned long long)maxStack);
-            if (P.parts == 0)
-            {
-                atomicAdd(&P.ctl->potential, pot);
-                if (P.sysPotential) atomicAdd(P.sysPotential + sys, pot);
-            }
             if (P.groupM2P) P.groupM2P[g] = nM2P;
             if (P.groupP2P) P.groupP2P[g] = nP2P;
         }
     }
 }
 
+// ------------------------------------------------------------------------------------------------ lists
+
+/*! the interaction list under construction, in items of P.itemWords words taken from the launch's pool as they are
+ *  needed. What an item holds depends on the walk alone, never on the order in which warps take items. */
+struct ListWriter
+{
+    int item;        // current item, -1 before the first
+    int count;       // items of the task
+    bool replicaSet; // the item knows the current replica
+    bool starved;    // the pool ran out
+    uint32_t pos;    // words used in the item
+    unsigned cost;   // interactions in the item: direct bodies + 2 x cells
+
+    //! room for a segment of @p payload words and @p segCost interactions (all lanes call it); false if starved
+    __device__ __forceinline__ bool room(const TraverseLaunch& P, unsigned g, uint32_t payload, unsigned segCost)
+    {
+        if (item < 0 || pos + 1 + kReplicaWords + payload > P.itemWords || (cost > 0 && cost + segCost > P.itemCost))
+        {
+            int next = 0;
+            if (laneId() == 0)
+            {
+                const unsigned at = atomicAdd(&P.ctl->itemCount, 1u);
+                next              = at < P.itemCapacity ? int(at) : -1;
+                if (next >= 0)
+                {
+                    if (item >= 0) P.items[item].words = pos;
+                    P.items[next] = ListItem{g, 0u, item, 0u};
+                }
+            }
+            next = __shfl_sync(0xffffffffu, next, 0);
+            if (next < 0)
+            {
+                starved = true;
+                return false;
+            }
+            item = next;
+            ++count;
+            replicaSet = false;
+            pos        = 0;
+            cost       = 0;
+        }
+        cost += segCost;
+        return true;
+    }
+
+    __device__ __forceinline__ uint32_t* at(const TraverseLaunch& P) const
+    {
+        return P.lists + size_t(item) * P.itemWords + pos;
+    }
+
+    //! the segments that follow are seen from the targets moved by replica @p rep
+    __device__ __forceinline__ void markReplica(const TraverseLaunch& P, const int rep[3])
+    {
+        if (replicaSet) return;
+        uint32_t* w = at(P);
+        if (laneId() == 0) w[0] = kSegReplica | (3u << 2);
+        if (laneId() < 3) w[1 + laneId()] = uint32_t(laneId() == 0 ? rep[0] : laneId() == 1 ? rep[1] : rep[2]);
+        pos += kReplicaWords;
+        replicaSet = true;
+    }
+
+    //! the first @p n (<= kM2PCap) pending cells as a segment; with @p images each cell's image follows, so that
+    //! cells of several replicas share a batch, which is seen from the targets where they are
+    __device__ __forceinline__ void cells(const TraverseLaunch& P, unsigned g, const WalkSmem& W, int n, bool images,
+                                          const int* rep)
+    {
+        const uint32_t payload = unsigned(images ? 2 * n : n);
+        if (!room(P, g, payload, 2u * unsigned(n))) return;
+        if (rep) markReplica(P, rep);
+        if (images) replicaSet = false;
+        uint32_t* w = at(P);
+        if (laneId() == 0) w[0] = (images ? kSegImages : kSegCells) | (uint32_t(n) << 2);
+        for (int k = int(laneId()); k < n; k += kWarp)
+        {
+            w[1 + k] = uint32_t(W.m2p[k]);
+            if (images) w[1 + n + k] = W.image[k];
+        }
+        pos += 1 + payload;
+    }
+
+    //! the first @p n (<= kSegLeafCap) pending leaves as a segment of (first body, body count) pairs
+    __device__ __forceinline__ void leaves(const TraverseLaunch& P, unsigned g, const WalkSmem& W, int n,
+                                           const int* rep)
+    {
+        const unsigned mine   = int(laneId()) < n ? unsigned(W.leaves[laneId()].y) : 0u;
+        const unsigned bodies = __reduce_add_sync(0xffffffffu, mine);
+        if (!room(P, g, 2u * unsigned(n), bodies)) return;
+        if (rep) markReplica(P, rep);
+        uint32_t* w    = at(P);
+        const int* src = reinterpret_cast<const int*>(W.leaves);
+        if (laneId() == 0) w[0] = kSegLeaves | (uint32_t(n) << 2);
+        for (int k = int(laneId()); k < 2 * n; k += kWarp)
+            w[1 + k] = uint32_t(src[k]);
+        pos += 1 + 2 * unsigned(n);
+    }
+};
+
+/*! walks the tree for one task and writes the interaction list to @p L: a group's whole walk, or part @p sub of
+ *  P.subWalks parts. False if the walk overflowed the stack or was starved. */
+template<class Nodes, class Targets>
+__device__ __forceinline__ bool walkTask(const TraverseLaunch& P, const Nodes& nodes, const Targets& tgt, unsigned g,
+                                         unsigned sub, WalkSmem& W, int* stack, ListWriter& L, unsigned& numM2P,
+                                         unsigned& numP2P, int& maxStack)
+{
+    const int lane    = laneId();
+    const unsigned lt = lanemaskLt();
+    const int b = int(P.groupStart[g]), e = int(P.groupEnd[g]);
+    float tc[3], ts[3];
+    {
+        float4 t0   = tgt.vec(min(b + lane, e - 1));
+        float4 t1   = tgt.vec(min(b + kWarp + lane, e - 1));
+        float lo[3] = {fminf(t0.x, t1.x), fminf(t0.y, t1.y), fminf(t0.z, t1.z)};
+        float hi[3] = {fmaxf(t0.x, t1.x), fmaxf(t0.y, t1.y), fmaxf(t0.z, t1.z)};
+#pragma unroll
+        for (int d = 0; d < 3; ++d)
+        {
+            float l = warpMin(lo[d]), h = warpMax(hi[d]);
+            tc[d]   = __fmul_rn(__fadd_rn(h, l), 0.5f);
+            ts[d]   = __fmul_rn(__fsub_rn(h, l), 0.5f);
+        }
+    }
+    GroupFrame F;
+    F.set(P, g);
+    // a part takes one child of the root, or in a periodic group every subWalks-th replica; a single-cell tree belongs
+    // to the first part
+    const int shells    = F.shells;
+    const bool replicas = shells > 0;
+    const bool images   = replicas && shells < kMaxImage;
+    const bool byChild  = P.subWalks > 1 && !replicas && F.rootEntry >= 0;
+    const int start     = byChild ? kRootOnly - (F.rootEntry + int(sub)) : F.rootEntry;
+    unsigned turn       = byChild ? 0u : P.subWalks - sub; // the replicas at multiples of subWalks are walked
+
+    L = ListWriter{-1, 0, false, false, 0u, 0u};
+    unsigned nM2P = 0, nP2P = 0; // of this lane
+    maxStack      = 0;
+    int nM        = 0;
+    bool overflow = false;
+    for (int iz = -shells; iz <= shells && !overflow; ++iz)
+        for (int iy = -shells; iy <= shells && !overflow; ++iy)
+            for (int ix = -shells; ix <= shells && !overflow; ++ix)
+            {
+                // the replica shift is added to and later subtracted from the group centre, as in the
+                // reference (traversal_gpu.cu:484-505), so the MAC decisions are the reference's. The targets
+                // are the original positions plus the shift: shifting them back and forth as the reference
+                // does leaves rounding residues, and a target then meets itself at about one float ulp of the
+                // box coordinates, which a softening below that turns into a large spurious force.
+                const float sh[3] = {__fmul_rn(float(ix), F.boxL[0]), __fmul_rn(float(iy), F.boxL[1]),
+                                     __fmul_rn(float(iz), F.boxL[2])};
+                const int rep[3]  = {ix, iy, iz};
+                L.replicaSet      = false;
+#pragma unroll
+                for (int d = 0; d < 3; ++d)
+                    tc[d] = __fadd_rn(tc[d], sh[d]);
+
+                int sp = turn % P.subWalks == 0 ? 1 : 0, nL = 0;
+                ++turn;
+                const uint32_t image = packImage(ix, iy, iz);
+                __syncwarp();
+                if (lane == 0) stack[0] = start;
+                __syncwarp();
+                while (sp > 0 && !L.starved)
+                {
+                    int k     = min(4, sp);
+                    sp -= k;
+                    int slot  = lane >> 3;
+                    int entry = slot < k ? stack[sp + slot] : -1;
+                    __syncwarp();
+                    int cell = -1;
+                    if (entry <= kRootOnly) cell = (lane & 7) == 0 ? kRootOnly - entry : -1;
+                    else if (entry >= 0) cell = entry + (lane & 7);
+
+                    bool valid = cell >= 0;
+                    float4 c   = make_float4(0.f, 0.f, 0.f, 0.f);
+                    int4 link  = make_int4(0, 0, 0, 0);
+                    if (valid) nodes.load(cell, c, link);
+                    bool close  = valid && macFails(c, tc, ts);
+                    bool isNode = link.x != 0;
+                    bool split  = close && isNode;
+                    unsigned bs = __ballot_sync(0xffffffffu, split);
+                    int nsplit  = __popc(bs);
+                    if (sp + nsplit > P.stackCapacity)
+                    {
+                        overflow = true;
+                        break;
+                    }
+                    if (split) stack[sp + __popc(bs & lt)] = link.x;
+                    sp += nsplit;
+                    maxStack = max(maxStack, sp);
+
+                    bool direct = close && !isNode;
+                    bool remote = direct && link.z == 0 && c.w != 0.f;
+                    bool approx = valid && (!close || remote);
+                    nM2P += approx ? 1u : 0u;
+
+                    bool evalM  = approx && c.w != 0.f; // massless cells contribute exactly zero
+                    unsigned bm = __ballot_sync(0xffffffffu, evalM);
+                    if (evalM)
+                    {
+                        W.m2p[nM + __popc(bm & lt)] = cell;
+                        if (images) W.image[nM + __popc(bm & lt)] = image;
+                    }
+                    nM += __popc(bm);
+
+                    bool hasB   = direct && link.z > 0;
+                    unsigned bl = __ballot_sync(0xffffffffu, hasB);
+                    if (hasB)
+                    {
+                        W.leaves[nL + __popc(bl & lt)] = make_int2(link.y, link.z);
+                        nP2P += unsigned(link.z);
+                    }
+                    nL += __popc(bl);
+                    __syncwarp();
+                    if (nM >= kM2PCap)
+                    {
+                        L.cells(P, g, W, kM2PCap, images, replicas && !images ? rep : nullptr);
+                        nM -= kM2PCap; // fewer than kWarp cells remain: one move per lane
+                        __syncwarp();
+                        if (lane < nM)
+                        {
+                            W.m2p[lane] = W.m2p[kM2PCap + lane];
+                            if (images) W.image[lane] = W.image[kM2PCap + lane];
+                        }
+                        __syncwarp();
+                    }
+                    if (nL >= kSegLeafCap)
+                    {
+                        L.leaves(P, g, W, kSegLeafCap, replicas ? rep : nullptr);
+                        nL -= kSegLeafCap;
+                        __syncwarp();
+                        if (lane < nL) W.leaves[lane] = W.leaves[kSegLeafCap + lane];
+                        __syncwarp();
+                    }
+                }
+                overflow |= L.starved;
+                if (nM > 0 && replicas && !images && !overflow)
+                {
+                    L.cells(P, g, W, nM, false, rep);
+                    nM = 0;
+                }
+                if (nL > 0 && !overflow) L.leaves(P, g, W, nL, replicas ? rep : nullptr);
+#pragma unroll
+                for (int d = 0; d < 3; ++d)
+                    tc[d] = __fsub_rn(tc[d], sh[d]);
+            }
+    if (nM > 0 && !overflow) L.cells(P, g, W, nM, images, nullptr);
+    numM2P = __reduce_add_sync(0xffffffffu, nM2P);
+    numP2P = __reduce_add_sync(0xffffffffu, nP2P);
+    return !overflow && !L.starved;
+}
+
+/*! walks the tree and writes the interaction lists. Warps take tasks from the queue: a group each, or one of P.subWalks
+ *  parts of a group's walk, so that a launch of few groups still fills the GPU. */
+template<class Nodes, class Targets>
+__global__ void __launch_bounds__(kTravThreads) walkKernel(TraverseLaunch P, Nodes nodes, Targets tgt)
+{
+    extern __shared__ __align__(16) unsigned char smemRaw[];
+    const int warp = threadIdx.x / kWarp, lane = laneId();
+    WalkSmem& W    = reinterpret_cast<WalkSmem*>(smemRaw)[warp];
+    int* stack     = reinterpret_cast<int*>(smemRaw + sizeof(WalkSmem) * kTravWarps) + warp * P.stackCapacity;
+    const unsigned numTasks = unsigned(P.numGroups) * P.subWalks;
+    while (true)
+    {
+        unsigned task = 0;
+        if (lane == 0) task = atomicAdd(&P.ctl->workCounter, 1u);
+        task = __shfl_sync(0xffffffffu, task, 0);
+        if (task >= numTasks) return;
+        const unsigned sub = task % P.subWalks;
+        const unsigned g   = P.groupList ? P.groupList[task / P.subWalks] : task / P.subWalks;
+        ListWriter L;
+        unsigned nM2P, nP2P;
+        int maxStack;
+        const bool ok = walkTask(P, nodes, tgt, g, sub, W, stack, L, nM2P, nP2P, maxStack);
+        __syncwarp();
+        if (lane != 0) continue;
+        P.taskLast[task] = L.item;
+        if (!L.starved) atomicMax(&P.ctl->stats[kMaxStack], (unsigned long long)maxStack);
+        if (!ok)
+        {
+            // nothing of this group is evaluated: it goes back to the host, to be walked again when the pool is free,
+            // or to be split when it overflowed the stack
+            if (atomicCAS(&P.groupState[g], 0u, L.starved ? kGroupUnserved : kGroupFailed) == 0u)
+            {
+                unsigned at = atomicAdd(L.starved ? &P.ctl->unservedCount : &P.ctl->failedCount, 1u);
+                (L.starved ? P.unservedGroups : P.failedGroups)[at] = g;
+            }
+            continue;
+        }
+        if (L.item >= 0)
+        {
+            P.items[L.item].words = L.pos;
+            P.items[L.item].only  = P.subWalks == 1 && L.count == 1 ? 1u : 0u;
+        }
+        if (P.subWalks > 1)
+        {
+            atomicAdd(&P.countM2P[g], nM2P);
+            atomicAdd(&P.countP2P[g], nP2P);
+        }
+        else
+        {
+            P.countM2P[g] = nM2P;
+            P.countP2P[g] = nP2P;
+        }
+    }
+}
+
+/*! evaluates the interaction lists. Warps take items from the queue; the sums of a group's only item are the group's
+ *  results, others go to P.partials for finishKernel. */
+template<class Nodes, class Targets, class Sources>
+__global__ void __launch_bounds__(kTravThreads, kEvalBlocks)
+    evalKernel(TraverseLaunch P, Nodes nodes, Targets tgt, Sources src)
+{
+    __shared__ WarpSmem smem[kTravWarps];
+    WarpSmem& S    = smem[threadIdx.x / kWarp];
+    const int lane = laneId();
+    const unsigned numItems = min(P.ctl->itemCount, P.itemCapacity);
+    while (true)
+    {
+        unsigned it = 0;
+        if (lane == 0) it = atomicAdd(&P.ctl->itemHead, 1u);
+        it = __shfl_sync(0xffffffffu, it, 0);
+        if (it >= numItems) return;
+        const ListItem item = P.items[it];
+        const unsigned g    = item.group;
+        if (P.groupState[g] != 0u) continue;
+        const int b = int(P.groupStart[g]), e = int(P.groupEnd[g]);
+        GroupFrame F;
+        F.set(P, g);
+        TargetState T;
+        float4 t0 = tgt.vec(min(b + lane, e - 1));
+        float4 t1 = tgt.vec(min(b + kWarp + lane, e - 1));
+        T.set(t0, t1);
+        T.h0       = __shfl_sync(0xffffffffu, t0.w, 0);
+        T.uniformH = __all_sync(0xffffffffu, t0.w == T.h0 && t1.w == T.h0);
+        setUniform(P, F, T, S);
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+            S.sums[0][c][lane] = S.sums[1][c][lane] = 0ull;
+
+        // a segment's header and its payload words l and l + 32 in lane l are loaded while the one before is evaluated
+        const uint32_t* w = P.lists + size_t(it) * P.itemWords;
+        uint32_t pos = 0, hdr = 0, w0 = 0, w1 = 0;
+        auto fetch = [&](uint32_t at)
+        {
+            if (at < item.words) hdr = __ldg(w + at);
+            if (at + 1 + lane < item.words) w0 = __ldg(w + at + 1 + lane);
+            if (at + 1 + kWarp + lane < item.words) w1 = __ldg(w + at + 1 + kWarp + lane);
+        };
+        fetch(0);
+        int nL = 0;
+        bool shifted = false; // T is the targets moved by a replica
+        while (true)
+        {
+            const bool end      = pos >= item.words;
+            const uint32_t kind = hdr & 3u;
+            const int n         = int(hdr >> 2);
+            const uint32_t c0 = w0, c1 = w1;
+            const uint32_t* payload = w + pos + 1;
+            pos += 1 + unsigned(kind == kSegLeaves || kind == kSegImages ? 2 * n : n);
+            fetch(pos);
+            __syncwarp();
+            if (!end && kind == kSegLeaves)
+            {
+                int* to = reinterpret_cast<int*>(S.leaves + nL);
+                if (lane < 2 * n) to[lane] = int(c0);
+                if (kWarp + lane < 2 * n) to[kWarp + lane] = int(c1);
+                nL += n;
+                __syncwarp();
+            }
+            // pending direct bodies are seen from T: all of them are summed before T moves
+            const bool moves = !end && (kind == kSegReplica || (kind == kSegImages && shifted));
+            if (nL > 0 && (end || moves || nL > kLeafCap - kWarp)) nL = evalP2P(S, nL, end || moves, src, T);
+            if (end) break;
+            if (moves)
+            {
+                float sh[3] = {0.f, 0.f, 0.f};
+                shifted     = false;
+                if (kind == kSegReplica)
+                {
+#pragma unroll
+                    for (int d = 0; d < 3; ++d)
+                    {
+                        const int r = int(__shfl_sync(0xffffffffu, c0, d));
+                        shifted |= r != 0;
+                        sh[d] = __fmul_rn(float(r), F.boxL[d]);
+                    }
+                }
+                t0 = tgt.vec(min(b + lane, e - 1));
+                t1 = tgt.vec(min(b + kWarp + lane, e - 1));
+                if (shifted)
+                {
+                    t0.x = __fadd_rn(t0.x, sh[0]), t1.x = __fadd_rn(t1.x, sh[0]);
+                    t0.y = __fadd_rn(t0.y, sh[1]), t1.y = __fadd_rn(t1.y, sh[1]);
+                    t0.z = __fadd_rn(t0.z, sh[2]), t1.z = __fadd_rn(t1.z, sh[2]);
+                }
+                T.set(t0, t1);
+            }
+            if (kind == kSegCells || kind == kSegImages)
+            {
+                if (lane < n) S.m2p[lane] = int(c0);
+                if (kWarp + lane < n) S.m2p[kWarp + lane] = int(c1);
+                if (kind == kSegImages)
+                {
+                    constexpr int kMB = m2pBatch<Nodes, true>();
+                    for (int k = lane; k < n; k += kWarp)
+                        S.image[k] = __ldg(payload + n + k);
+                    __syncwarp();
+                    for (int k = 0; k < n; k += kMB)
+                        evalM2P<true>(S, k, min(kMB, n - k), nodes, T, F.boxL);
+                }
+                else
+                {
+                    constexpr int kMB = m2pBatch<Nodes>();
+                    __syncwarp();
+                    for (int k = 0; k < n; k += kMB)
+                        evalM2P(S, k, min(kMB, n - k), nodes, T);
+                }
+            }
+        }
+        const ListSums r = readSums(S);
+        __syncwarp();
+        if (item.only) storeGroup(P, tgt, r, b, e, F.sys);
+        else
+        {
+            float4* out       = P.partials + size_t(it) * (2 * kWarp);
+            out[lane]         = make_float4(r.phi[0], r.x[0], r.y[0], r.z[0]);
+            out[kWarp + lane] = make_float4(r.phi[1], r.x[1], r.y[1], r.z[1]);
+        }
+    }
+}
+
+constexpr int kFinishThreads = 256;
+
+/*! every group of the launch, one warp each: interaction counts and statistics, and the results of the groups whose
+ *  list became items (or is empty): the items' sums added in FP64 in a fixed order */
+template<class Targets>
+__global__ void __launch_bounds__(kFinishThreads) finishKernel(TraverseLaunch P, Targets tgt)
+{
+    const int lane        = laneId();
+    const unsigned stride = gridDim.x * (kFinishThreads / kWarp);
+    unsigned long long sumP = 0, sumM = 0, maxP = 0, maxM = 0;
+    for (unsigned i = (blockIdx.x * kFinishThreads + threadIdx.x) / kWarp; i < unsigned(P.numGroups); i += stride)
+    {
+        const unsigned g = P.groupList ? P.groupList[i] : i;
+        if (P.groupState[g] != 0u) continue;
+        const int b = int(P.groupStart[g]), e = int(P.groupEnd[g]);
+        const unsigned nM = P.countM2P[g], nP = P.countP2P[g];
+        sumP += (unsigned long long)nP * unsigned(e - b);
+        sumM += (unsigned long long)nM * unsigned(e - b);
+        maxP = max(maxP, (unsigned long long)nP);
+        maxM = max(maxM, (unsigned long long)nM);
+        if (lane == 0 && P.groupM2P) P.groupM2P[g] = nM;
+        if (lane == 0 && P.groupP2P) P.groupP2P[g] = nP;
+        double sum[2][4] = {};
+        const int last   = P.taskLast[i * P.subWalks];
+        if (last >= 0 && P.items[last].only) continue;
+        for (unsigned sub = 0; sub < P.subWalks; ++sub)
+        {
+            for (int it = P.taskLast[i * P.subWalks + sub]; it >= 0; it = P.items[it].prev)
+            {
+#pragma unroll
+                for (int t = 0; t < 2; ++t)
+                {
+                    float4 v = P.partials[size_t(it) * (2 * kWarp) + t * kWarp + lane];
+                    sum[t][0] += v.x;
+                    sum[t][1] += v.y;
+                    sum[t][2] += v.z;
+                    sum[t][3] += v.w;
+                }
+            }
+        }
+        double pot = 0.0;
+#pragma unroll
+        for (int t = 0; t < 2; ++t)
+        {
+            int idx = b + t * kWarp + lane;
+            if (idx < e)
+            {
+                float phi = float(sum[t][0]), gx = float(sum[t][1]), gy = float(sum[t][2]), gz = float(sum[t][3]);
+                float mi  = tgt.scalar(idx);
+                pot += double(mi) * double(phi);
+                storeResult(P, idx, P.G * mi * phi, P.G * gx, P.G * gy, P.G * gz);
+            }
+        }
+        pot = warpSum(pot);
+        if (lane == 0)
+        {
+            atomicAdd(&P.ctl->potential, pot);
+            if (P.sysPotential) atomicAdd(P.sysPotential + (P.groupSys ? P.groupSys[g] : 0u), pot);
+        }
+    }
+    // every lane of a warp holds the same counts; one set of atomics per block
+    __shared__ unsigned long long sh[4][kFinishThreads / kWarp];
+    const int warp = threadIdx.x / kWarp;
+    if (lane == 0) sh[0][warp] = sumP, sh[1][warp] = sumM, sh[2][warp] = maxP, sh[3][warp] = maxM;
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    for (int k = 1; k < kFinishThreads / kWarp; ++k)
+    {
+        sumP += sh[0][k];
+        sumM += sh[1][k];
+        maxP = max(maxP, sh[2][k]);
+        maxM = max(maxM, sh[3][k]);
+    }
+    if (sumP == 0 && sumM == 0) return;
+    atomicAdd(&P.ctl->stats[kSumP2P], sumP);
+    atomicMax(&P.ctl->stats[kMaxP2P], maxP);
+    atomicAdd(&P.ctl->stats[kSumM2P], sumM);
+    atomicMax(&P.ctl->stats[kMaxM2P], maxM);
+}
+
 template<class Nodes, class Targets, class Sources>
 static void launchTyped(const TraverseLaunch& t, const Nodes& nodes, const Targets& tgt, const Sources& src,
                         int smCount, cudaStream_t s)
 {
-    auto kernel = t.parts > 0 ? traverseKernel<Nodes, Targets, Sources, true>
-                              : traverseKernel<Nodes, Targets, Sources, false>;
-    size_t smem = sizeof(int) * kTravWarps * size_t(t.stackCapacity) + sizeof(WarpSmem) * kTravWarps;
-    RYO_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
-    int perSm = 0;
-    RYO_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, kernel, kTravThreads, smem));
-    if (perSm < 1) perSm = 1;
-    int items  = t.parts > 0 ? int(t.numHeavy) * t.parts : t.numGroups;
-    int want   = (items + kTravWarps - 1) / kTravWarps;
-    int blocks = min(want, perSm * smCount);
-    kernel<<<blocks, kTravThreads, smem, s>>>(t, nodes, tgt, src);
+    auto blocksFor = [&](auto kernel, size_t smem, size_t warps)
+    {
+        int perSm = 0;
+        RYO_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+        RYO_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, kernel, kTravThreads, smem));
+        return unsigned(std::min((warps + kTravWarps - 1) / kTravWarps, size_t(std::max(perSm, 1)) * smCount));
+    };
+    const size_t stack = sizeof(int) * kTravWarps * size_t(t.stackCapacity);
+    if (t.subWalks == 0)
+    {
+        auto kernel       = traverseKernel<Nodes, Targets, Sources>;
+        const size_t smem = stack + sizeof(WarpSmem) * kTravWarps;
+        kernel<<<blocksFor(kernel, smem, size_t(t.numGroups)), kTravThreads, smem, s>>>(t, nodes, tgt, src);
+        RYO_LAUNCH_CHECK();
+        return;
+    }
+    auto walk         = walkKernel<Nodes, Targets>;
+    auto eval         = evalKernel<Nodes, Targets, Sources>;
+    const size_t smem = stack + sizeof(WalkSmem) * kTravWarps;
+    walk<<<blocksFor(walk, smem, size_t(t.numGroups) * t.subWalks), kTravThreads, smem, s>>>(t, nodes, tgt);
+    RYO_LAUNCH_CHECK();
+    eval<<<blocksFor(eval, 0, size_t(t.itemCapacity)), kTravThreads, 0, s>>>(t, nodes, tgt, src);
+    RYO_LAUNCH_CHECK();
+    const size_t fin = ceilDiv(size_t(t.numGroups) * kWarp, kFinishThreads);
+    finishKernel<<<unsigned(std::min(fin, size_t(8) * smCount)), kFinishThreads, 0, s>>>(t, tgt);
     RYO_LAUNCH_CHECK();
 }
 
 void launchTraverse(const TraverseLaunch& t, int smCount, cudaStream_t s)
 {
-    if (t.numGroups <= 0 || (t.parts > 0 && t.numHeavy == 0)) return;
+    if (t.numGroups <= 0) return;
     if (t.precision != kPrecisionF32)
     {
         launchTraverse64(t, smCount, s);
