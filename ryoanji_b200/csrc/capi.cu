@@ -613,12 +613,13 @@ void traverseLists(ryo_ctx* ctx, TraverseLaunch t, const uint32_t* list, uint32_
     RYO_CUDA(cudaMemsetAsync(t.groupState, 0, 3 * sizeof(uint32_t) * size_t(numGroups), s));
     uint32_t* unserved[2] = {ctx->scratch<uint32_t>("trav.unservedA", count, s),
                              ctx->scratch<uint32_t>("trav.unservedB", count, s)};
-    uint32_t chunk        = count; // groups per launch
+    uint32_t chunk         = count; // groups per launch
+    const size_t perTarget = t.precision == kPrecisionF32 ? 1 : 2; // float4 per target's sums
     for (int flip = 0;; flip ^= 1)
     {
         t.items      = ctx->scratch<ListItem>("trav.items", t.itemCapacity, s);
         t.lists      = ctx->scratch<uint32_t>("trav.lists", size_t(t.itemCapacity) * t.itemWords, s);
-        t.partials   = ctx->scratch<float4>("trav.partials", size_t(t.itemCapacity) * 2 * kWarp, s);
+        t.partials   = ctx->scratch<float4>("trav.partials", size_t(t.itemCapacity) * 2 * kWarp * perTarget, s);
         uint32_t left = 0;
         for (uint32_t first = 0; first < count; first += chunk)
         {
@@ -663,7 +664,7 @@ void runTraversal(ryo_ctx* ctx, TraverseLaunch t, cudaStream_t s, double* potent
     {
         if (pass > 0) launchTraversalReset(ctx->ctl, kTravPass, s);
         ++pass;
-        if (t.precision == kPrecisionF32 && solveGroups <= kListGroups)
+        if (solveGroups <= kListGroups)
             traverseLists(ctx, t, nullptr, uint32_t(t.numGroups), solveGroups, ownStack, hc, s);
         else
         {

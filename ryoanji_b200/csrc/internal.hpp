@@ -373,7 +373,7 @@ struct TraverseLaunch
     const uint32_t* groupList;
     ListItem* items;
     uint32_t* lists;
-    float4* partials;       // (-phi, ax, ay, az) of an item's 64 targets
+    float4* partials;       // (phi, ax, ay, az) of an item's 64 targets; doubles for double coordinates
     uint32_t itemCapacity, itemWords;
     unsigned itemCost;
     int* taskLast;          // per part of a walk: its last item, -1 if its list is empty

@@ -33,33 +33,14 @@
  *     sums and compensations live in shared memory, which keeps the kernel at 96 registers (five blocks per SM);
  *   - the MAC test uses explicitly rounded single operations so that every decision is reproducible bit for bit.
  */
-#include "internal.hpp"
+#include "lists.cuh"
 
 namespace ryo
 {
 
-constexpr int kTravWarps    = 4;
-constexpr int kTravThreads  = kTravWarps * kWarp;
-constexpr int kM2PCap       = 64;  // pending approximated cells (flushed at 64, or 32 for dipole expansions)
 constexpr int kLeafCap      = 64;  // pending direct leaves (flushed when more than 32 are pending)
 constexpr int kP2PBatch     = 2 * kWarp; // direct bodies evaluated per staging round (two per lane)
 constexpr int kEvalBlocks   = 5;     // resident blocks of the list evaluation per SM (4: 1-2% slower, 6: 2-3%)
-constexpr int kSegLeafCap   = kWarp; // direct leaves per list segment
-constexpr int kRootOnly     = -2;  // stack marker: the root itself is the only cell (single-leaf tree); a marker
-                                   // -(r + 2) stands for the single cell r
-
-// segment header of an interaction list: kind in the low two bits, entry count above
-constexpr uint32_t kSegCells = 0, kSegLeaves = 1, kSegReplica = 2, kSegImages = 3;
-constexpr int kReplicaWords  = 4;
-
-//! a list walk's pending entries: a segment leaves fewer than a segment's, and one walk step adds at most kWarp
-struct WalkSmem
-{
-    int m2p[kM2PCap + kWarp];
-    uint32_t image[kM2PCap + kWarp]; // of periodic groups: the image each pending cell is seen in
-    int2 leaves[kSegLeafCap + kWarp];
-};
-
 struct WarpSmem
 {
     int m2p[kM2PCap + kWarp];
@@ -279,6 +260,8 @@ __device__ __forceinline__ Acc2 zero2()
 //! node data from the packed 64-byte records of the solver path
 struct RecordNodes
 {
+    using Real   = float;
+    using Center = float4;
     static constexpr bool kDipole = false;
     const NodeRecord* __restrict__ r;
     __device__ __forceinline__ void load(int cell, float4& c, int4& link) const
@@ -309,6 +292,8 @@ struct RecordNodesMDQ : RecordNodes
 //! node data from the reference's separate arrays (centres, multipoles, childOffsets, internalToLeaf, layout)
 struct ArrayNodes
 {
+    using Real   = float;
+    using Center = float4;
     static constexpr bool kDipole = false;
     const float4* __restrict__ centers;
     const float4* __restrict__ mpoles; // two float4 per node (three for CartesianMDQpole)
@@ -355,6 +340,11 @@ struct PackedBodies
     const float4* __restrict__ xyzw;
     const float* __restrict__ s;
     __device__ __forceinline__ float4 vec(int i) const { return __ldg(xyzw + i); }
+    __device__ __forceinline__ void position(int i, float p[3]) const
+    {
+        const float4 v = vec(i);
+        p[0] = v.x, p[1] = v.y, p[2] = v.z;
+    }
     __device__ __forceinline__ float scalar(int i) const { return __ldg(s + i); }
 };
 
@@ -369,6 +359,10 @@ struct SoABodies
     __device__ __forceinline__ float4 vec(int i) const
     {
         return make_float4(__ldg(x + i), __ldg(y + i), __ldg(z + i), __ldg(w + i));
+    }
+    __device__ __forceinline__ void position(int i, float p[3]) const
+    {
+        p[0] = __ldg(x + i), p[1] = __ldg(y + i), p[2] = __ldg(z + i);
     }
     __device__ __forceinline__ float scalar(int i) const { return __ldg(s + i); }
 };
@@ -395,17 +389,6 @@ __device__ __forceinline__ void addBatchS(WarpSmem& S, const Acc2& part)
         S.sums[0][c][lane] = sum;
         S.sums[1][c][lane] = comp;
     }
-}
-
-//! a periodic image (ix, iy, iz), each in [-kMaxImage, kMaxImage), in one word, and its components
-constexpr int kMaxImage = 512;
-__device__ __forceinline__ uint32_t packImage(int ix, int iy, int iz)
-{
-    return uint32_t(ix + kMaxImage) | (uint32_t(iy + kMaxImage) << 10) | (uint32_t(iz + kMaxImage) << 20);
-}
-__device__ __forceinline__ float imageShift(uint32_t image, int d)
-{
-    return float(int((image >> (10 * d)) & 1023u) - kMaxImage);
 }
 
 //! approximated cells per evaluation batch: 64 quadrupoles (5 staged float4 each), or 32 dipole expansions (7) or
@@ -743,40 +726,9 @@ __device__ __forceinline__ void storeResult(const TraverseLaunch& P, int idx, fl
     P.az[idx] = (add ? P.az[idx] : 0.f) + z;
 }
 
-//! the tree root and periodic images of a group: the launch's, or its system's in a batched solve
-struct GroupFrame
-{
-    int rootEntry, shells;
-    float boxL[3];
-    uint32_t sys;
-
-    __device__ __forceinline__ void set(const TraverseLaunch& P, unsigned g)
-    {
-        rootEntry = P.numNodes == 1 ? kRootOnly : P.initNode;
-        shells    = P.numShells;
-        sys       = 0;
-        if (P.groupSys)
-        {
-            sys               = P.groupSys[g];
-            const SysTrav& st = P.systems[sys];
-            rootEntry         = st.entry;
-            shells            = st.numShells;
-#pragma unroll
-            for (int d = 0; d < 3; ++d)
-                boxL[d] = st.boxL[d];
-        }
-        else
-        {
-#pragma unroll
-            for (int d = 0; d < 3; ++d)
-                boxL[d] = P.boxL[d];
-        }
-    }
-};
-
 //! whether the targets' softening, and the sources' mass, are one for all bodies: those of the launch, or in a batched
 //! solve the system's, whose groups meet only its own bodies
-__device__ __forceinline__ void setUniform(const TraverseLaunch& P, const GroupFrame& F, const TargetState& T,
+__device__ __forceinline__ void setUniform(const TraverseLaunch& P, const GroupFrame<float>& F, const TargetState& T,
                                            WarpSmem& S)
 {
     if (laneId() != 0) return;
@@ -881,7 +833,7 @@ __global__ void __launch_bounds__(kTravThreads, 5)
             ts[d]   = __fmul_rn(__fsub_rn(h, l), 0.5f);
         }
 
-        GroupFrame F;
+        GroupFrame<float> F;
         F.set(P, g);
         setUniform(P, F, T, S);
 
@@ -1024,311 +976,6 @@ __global__ void __launch_bounds__(kTravThreads, 5)
     }
 }
 
-// ------------------------------------------------------------------------------------------------ lists
-
-/*! the interaction list under construction, in items of P.itemWords words taken from the launch's pool as they are
- *  needed. What an item holds depends on the walk alone, never on the order in which warps take items. */
-struct ListWriter
-{
-    int item;        // current item, -1 before the first
-    int count;       // items of the task
-    bool replicaSet; // the item knows the current replica
-    bool starved;    // the pool ran out
-    uint32_t pos;    // words used in the item
-    unsigned cost;   // interactions in the item: direct bodies + 2 x cells
-
-    //! room for a segment of @p payload words and @p segCost interactions (all lanes call it); false if starved
-    __device__ __forceinline__ bool room(const TraverseLaunch& P, unsigned g, uint32_t payload, unsigned segCost)
-    {
-        if (item < 0 || pos + 1 + kReplicaWords + payload > P.itemWords || (cost > 0 && cost + segCost > P.itemCost))
-        {
-            int next = 0;
-            if (laneId() == 0)
-            {
-                const unsigned at = atomicAdd(&P.ctl->itemCount, 1u);
-                next              = at < P.itemCapacity ? int(at) : -1;
-                if (next >= 0)
-                {
-                    if (item >= 0) P.items[item].words = pos;
-                    P.items[next] = ListItem{g, 0u, item, 0u};
-                }
-            }
-            next = __shfl_sync(0xffffffffu, next, 0);
-            if (next < 0)
-            {
-                starved = true;
-                return false;
-            }
-            item = next;
-            ++count;
-            replicaSet = false;
-            pos        = 0;
-            cost       = 0;
-        }
-        cost += segCost;
-        return true;
-    }
-
-    __device__ __forceinline__ uint32_t* at(const TraverseLaunch& P) const
-    {
-        return P.lists + size_t(item) * P.itemWords + pos;
-    }
-
-    //! the segments that follow are seen from the targets moved by replica @p rep
-    __device__ __forceinline__ void markReplica(const TraverseLaunch& P, const int rep[3])
-    {
-        if (replicaSet) return;
-        uint32_t* w = at(P);
-        if (laneId() == 0) w[0] = kSegReplica | (3u << 2);
-        if (laneId() < 3) w[1 + laneId()] = uint32_t(laneId() == 0 ? rep[0] : laneId() == 1 ? rep[1] : rep[2]);
-        pos += kReplicaWords;
-        replicaSet = true;
-    }
-
-    //! the first @p n (<= kM2PCap) pending cells as a segment; with @p images each cell's image follows, so that
-    //! cells of several replicas share a batch, which is seen from the targets where they are
-    __device__ __forceinline__ void cells(const TraverseLaunch& P, unsigned g, const WalkSmem& W, int n, bool images,
-                                          const int* rep)
-    {
-        const uint32_t payload = unsigned(images ? 2 * n : n);
-        if (!room(P, g, payload, 2u * unsigned(n))) return;
-        if (rep) markReplica(P, rep);
-        if (images) replicaSet = false;
-        uint32_t* w = at(P);
-        if (laneId() == 0) w[0] = (images ? kSegImages : kSegCells) | (uint32_t(n) << 2);
-        for (int k = int(laneId()); k < n; k += kWarp)
-        {
-            w[1 + k] = uint32_t(W.m2p[k]);
-            if (images) w[1 + n + k] = W.image[k];
-        }
-        pos += 1 + payload;
-    }
-
-    //! the first @p n (<= kSegLeafCap) pending leaves as a segment of (first body, body count) pairs
-    __device__ __forceinline__ void leaves(const TraverseLaunch& P, unsigned g, const WalkSmem& W, int n,
-                                           const int* rep)
-    {
-        const unsigned mine   = int(laneId()) < n ? unsigned(W.leaves[laneId()].y) : 0u;
-        const unsigned bodies = __reduce_add_sync(0xffffffffu, mine);
-        if (!room(P, g, 2u * unsigned(n), bodies)) return;
-        if (rep) markReplica(P, rep);
-        uint32_t* w    = at(P);
-        const int* src = reinterpret_cast<const int*>(W.leaves);
-        if (laneId() == 0) w[0] = kSegLeaves | (uint32_t(n) << 2);
-        for (int k = int(laneId()); k < 2 * n; k += kWarp)
-            w[1 + k] = uint32_t(src[k]);
-        pos += 1 + 2 * unsigned(n);
-    }
-};
-
-/*! walks the tree for one task and writes the interaction list to @p L: a group's whole walk, or part @p sub of
- *  P.subWalks parts. False if the walk overflowed the stack or was starved. */
-template<class Nodes, class Targets>
-__device__ __forceinline__ bool walkTask(const TraverseLaunch& P, const Nodes& nodes, const Targets& tgt, unsigned g,
-                                         unsigned sub, WalkSmem& W, int* stack, ListWriter& L, unsigned& numM2P,
-                                         unsigned& numP2P, int& maxStack)
-{
-    const int lane    = laneId();
-    const unsigned lt = lanemaskLt();
-    const int b = int(P.groupStart[g]), e = int(P.groupEnd[g]);
-    float tc[3], ts[3];
-    {
-        float4 t0   = tgt.vec(min(b + lane, e - 1));
-        float4 t1   = tgt.vec(min(b + kWarp + lane, e - 1));
-        float lo[3] = {fminf(t0.x, t1.x), fminf(t0.y, t1.y), fminf(t0.z, t1.z)};
-        float hi[3] = {fmaxf(t0.x, t1.x), fmaxf(t0.y, t1.y), fmaxf(t0.z, t1.z)};
-#pragma unroll
-        for (int d = 0; d < 3; ++d)
-        {
-            float l = warpMin(lo[d]), h = warpMax(hi[d]);
-            tc[d]   = __fmul_rn(__fadd_rn(h, l), 0.5f);
-            ts[d]   = __fmul_rn(__fsub_rn(h, l), 0.5f);
-        }
-    }
-    GroupFrame F;
-    F.set(P, g);
-    // a part takes one child of the root, or in a periodic group every subWalks-th replica; a single-cell tree belongs
-    // to the first part
-    const int shells    = F.shells;
-    const bool replicas = shells > 0;
-    const bool images   = replicas && shells < kMaxImage;
-    const bool byChild  = P.subWalks > 1 && !replicas && F.rootEntry >= 0;
-    const int start     = byChild ? kRootOnly - (F.rootEntry + int(sub)) : F.rootEntry;
-    unsigned turn       = byChild ? 0u : P.subWalks - sub; // the replicas at multiples of subWalks are walked
-
-    L = ListWriter{-1, 0, false, false, 0u, 0u};
-    unsigned nM2P = 0, nP2P = 0; // of this lane
-    maxStack      = 0;
-    int nM        = 0;
-    bool overflow = false;
-    for (int iz = -shells; iz <= shells && !overflow; ++iz)
-        for (int iy = -shells; iy <= shells && !overflow; ++iy)
-            for (int ix = -shells; ix <= shells && !overflow; ++ix)
-            {
-                // the replica shift is added to and later subtracted from the group centre, as in the
-                // reference (traversal_gpu.cu:484-505), so the MAC decisions are the reference's. The targets
-                // are the original positions plus the shift: shifting them back and forth as the reference
-                // does leaves rounding residues, and a target then meets itself at about one float ulp of the
-                // box coordinates, which a softening below that turns into a large spurious force.
-                const float sh[3] = {__fmul_rn(float(ix), F.boxL[0]), __fmul_rn(float(iy), F.boxL[1]),
-                                     __fmul_rn(float(iz), F.boxL[2])};
-                const int rep[3]  = {ix, iy, iz};
-                L.replicaSet      = false;
-#pragma unroll
-                for (int d = 0; d < 3; ++d)
-                    tc[d] = __fadd_rn(tc[d], sh[d]);
-
-                int sp = turn % P.subWalks == 0 ? 1 : 0, nL = 0;
-                ++turn;
-                const uint32_t image = packImage(ix, iy, iz);
-                __syncwarp();
-                if (lane == 0) stack[0] = start;
-                __syncwarp();
-                while (sp > 0 && !L.starved)
-                {
-                    int k     = min(4, sp);
-                    sp -= k;
-                    int slot  = lane >> 3;
-                    int entry = slot < k ? stack[sp + slot] : -1;
-                    __syncwarp();
-                    int cell = -1;
-                    if (entry <= kRootOnly) cell = (lane & 7) == 0 ? kRootOnly - entry : -1;
-                    else if (entry >= 0) cell = entry + (lane & 7);
-
-                    bool valid = cell >= 0;
-                    float4 c   = make_float4(0.f, 0.f, 0.f, 0.f);
-                    int4 link  = make_int4(0, 0, 0, 0);
-                    if (valid) nodes.load(cell, c, link);
-                    bool close  = valid && macFails(c, tc, ts);
-                    bool isNode = link.x != 0;
-                    bool split  = close && isNode;
-                    unsigned bs = __ballot_sync(0xffffffffu, split);
-                    int nsplit  = __popc(bs);
-                    if (sp + nsplit > P.stackCapacity)
-                    {
-                        overflow = true;
-                        break;
-                    }
-                    if (split) stack[sp + __popc(bs & lt)] = link.x;
-                    sp += nsplit;
-                    maxStack = max(maxStack, sp);
-
-                    bool direct = close && !isNode;
-                    bool remote = direct && link.z == 0 && c.w != 0.f;
-                    bool approx = valid && (!close || remote);
-                    nM2P += approx ? 1u : 0u;
-
-                    bool evalM  = approx && c.w != 0.f; // massless cells contribute exactly zero
-                    unsigned bm = __ballot_sync(0xffffffffu, evalM);
-                    if (evalM)
-                    {
-                        W.m2p[nM + __popc(bm & lt)] = cell;
-                        if (images) W.image[nM + __popc(bm & lt)] = image;
-                    }
-                    nM += __popc(bm);
-
-                    bool hasB   = direct && link.z > 0;
-                    unsigned bl = __ballot_sync(0xffffffffu, hasB);
-                    if (hasB)
-                    {
-                        W.leaves[nL + __popc(bl & lt)] = make_int2(link.y, link.z);
-                        nP2P += unsigned(link.z);
-                    }
-                    nL += __popc(bl);
-                    __syncwarp();
-                    if (nM >= kM2PCap)
-                    {
-                        L.cells(P, g, W, kM2PCap, images, replicas && !images ? rep : nullptr);
-                        nM -= kM2PCap; // fewer than kWarp cells remain: one move per lane
-                        __syncwarp();
-                        if (lane < nM)
-                        {
-                            W.m2p[lane] = W.m2p[kM2PCap + lane];
-                            if (images) W.image[lane] = W.image[kM2PCap + lane];
-                        }
-                        __syncwarp();
-                    }
-                    if (nL >= kSegLeafCap)
-                    {
-                        L.leaves(P, g, W, kSegLeafCap, replicas ? rep : nullptr);
-                        nL -= kSegLeafCap;
-                        __syncwarp();
-                        if (lane < nL) W.leaves[lane] = W.leaves[kSegLeafCap + lane];
-                        __syncwarp();
-                    }
-                }
-                overflow |= L.starved;
-                if (nM > 0 && replicas && !images && !overflow)
-                {
-                    L.cells(P, g, W, nM, false, rep);
-                    nM = 0;
-                }
-                if (nL > 0 && !overflow) L.leaves(P, g, W, nL, replicas ? rep : nullptr);
-#pragma unroll
-                for (int d = 0; d < 3; ++d)
-                    tc[d] = __fsub_rn(tc[d], sh[d]);
-            }
-    if (nM > 0 && !overflow) L.cells(P, g, W, nM, images, nullptr);
-    numM2P = __reduce_add_sync(0xffffffffu, nM2P);
-    numP2P = __reduce_add_sync(0xffffffffu, nP2P);
-    return !overflow && !L.starved;
-}
-
-/*! walks the tree and writes the interaction lists. Warps take tasks from the queue: a group each, or one of P.subWalks
- *  parts of a group's walk, so that a launch of few groups still fills the GPU. */
-template<class Nodes, class Targets>
-__global__ void __launch_bounds__(kTravThreads) walkKernel(TraverseLaunch P, Nodes nodes, Targets tgt)
-{
-    extern __shared__ __align__(16) unsigned char smemRaw[];
-    const int warp = threadIdx.x / kWarp, lane = laneId();
-    WalkSmem& W    = reinterpret_cast<WalkSmem*>(smemRaw)[warp];
-    int* stack     = reinterpret_cast<int*>(smemRaw + sizeof(WalkSmem) * kTravWarps) + warp * P.stackCapacity;
-    const unsigned numTasks = unsigned(P.numGroups) * P.subWalks;
-    while (true)
-    {
-        unsigned task = 0;
-        if (lane == 0) task = atomicAdd(&P.ctl->workCounter, 1u);
-        task = __shfl_sync(0xffffffffu, task, 0);
-        if (task >= numTasks) return;
-        const unsigned sub = task % P.subWalks;
-        const unsigned g   = P.groupList ? P.groupList[task / P.subWalks] : task / P.subWalks;
-        ListWriter L;
-        unsigned nM2P, nP2P;
-        int maxStack;
-        const bool ok = walkTask(P, nodes, tgt, g, sub, W, stack, L, nM2P, nP2P, maxStack);
-        __syncwarp();
-        if (lane != 0) continue;
-        P.taskLast[task] = L.item;
-        if (!L.starved) atomicMax(&P.ctl->stats[kMaxStack], (unsigned long long)maxStack);
-        if (!ok)
-        {
-            // nothing of this group is evaluated: it goes back to the host, to be walked again when the pool is free,
-            // or to be split when it overflowed the stack
-            if (atomicCAS(&P.groupState[g], 0u, L.starved ? kGroupUnserved : kGroupFailed) == 0u)
-            {
-                unsigned at = atomicAdd(L.starved ? &P.ctl->unservedCount : &P.ctl->failedCount, 1u);
-                (L.starved ? P.unservedGroups : P.failedGroups)[at] = g;
-            }
-            continue;
-        }
-        if (L.item >= 0)
-        {
-            P.items[L.item].words = L.pos;
-            P.items[L.item].only  = P.subWalks == 1 && L.count == 1 ? 1u : 0u;
-        }
-        if (P.subWalks > 1)
-        {
-            atomicAdd(&P.countM2P[g], nM2P);
-            atomicAdd(&P.countP2P[g], nP2P);
-        }
-        else
-        {
-            P.countM2P[g] = nM2P;
-            P.countP2P[g] = nP2P;
-        }
-    }
-}
-
 /*! evaluates the interaction lists. Warps take items from the queue; the sums of a group's only item are the group's
  *  results, others go to P.partials for finishKernel. */
 template<class Nodes, class Targets, class Sources>
@@ -1349,7 +996,7 @@ __global__ void __launch_bounds__(kTravThreads, kEvalBlocks)
         const unsigned g    = item.group;
         if (P.groupState[g] != 0u) continue;
         const int b = int(P.groupStart[g]), e = int(P.groupEnd[g]);
-        GroupFrame F;
+        GroupFrame<float> F;
         F.set(P, g);
         TargetState T;
         float4 t0 = tgt.vec(min(b + lane, e - 1));
@@ -1454,116 +1101,38 @@ __global__ void __launch_bounds__(kTravThreads, kEvalBlocks)
     }
 }
 
-constexpr int kFinishThreads = 256;
-
-/*! every group of the launch, one warp each: interaction counts and statistics, and the results of the groups whose
- *  list became items (or is empty): the items' sums added in FP64 in a fixed order */
+//! finishKernel's sums and results
 template<class Targets>
-__global__ void __launch_bounds__(kFinishThreads) finishKernel(TraverseLaunch P, Targets tgt)
+struct FloatSink
 {
-    const int lane        = laneId();
-    const unsigned stride = gridDim.x * (kFinishThreads / kWarp);
-    unsigned long long sumP = 0, sumM = 0, maxP = 0, maxM = 0;
-    for (unsigned i = (blockIdx.x * kFinishThreads + threadIdx.x) / kWarp; i < unsigned(P.numGroups); i += stride)
+    Targets tgt;
+    __device__ __forceinline__ float4 part(const TraverseLaunch& P, size_t i) const { return P.partials[i]; }
+    __device__ __forceinline__ double store(const TraverseLaunch& P, int idx, const double s[4]) const
     {
-        const unsigned g = P.groupList ? P.groupList[i] : i;
-        if (P.groupState[g] != 0u) continue;
-        const int b = int(P.groupStart[g]), e = int(P.groupEnd[g]);
-        const unsigned nM = P.countM2P[g], nP = P.countP2P[g];
-        sumP += (unsigned long long)nP * unsigned(e - b);
-        sumM += (unsigned long long)nM * unsigned(e - b);
-        maxP = max(maxP, (unsigned long long)nP);
-        maxM = max(maxM, (unsigned long long)nM);
-        if (lane == 0 && P.groupM2P) P.groupM2P[g] = nM;
-        if (lane == 0 && P.groupP2P) P.groupP2P[g] = nP;
-        double sum[2][4] = {};
-        const int last   = P.taskLast[i * P.subWalks];
-        if (last >= 0 && P.items[last].only) continue;
-        for (unsigned sub = 0; sub < P.subWalks; ++sub)
-        {
-            for (int it = P.taskLast[i * P.subWalks + sub]; it >= 0; it = P.items[it].prev)
-            {
-#pragma unroll
-                for (int t = 0; t < 2; ++t)
-                {
-                    float4 v = P.partials[size_t(it) * (2 * kWarp) + t * kWarp + lane];
-                    sum[t][0] += v.x;
-                    sum[t][1] += v.y;
-                    sum[t][2] += v.z;
-                    sum[t][3] += v.w;
-                }
-            }
-        }
-        double pot = 0.0;
-#pragma unroll
-        for (int t = 0; t < 2; ++t)
-        {
-            int idx = b + t * kWarp + lane;
-            if (idx < e)
-            {
-                float phi = float(sum[t][0]), gx = float(sum[t][1]), gy = float(sum[t][2]), gz = float(sum[t][3]);
-                float mi  = tgt.scalar(idx);
-                pot += double(mi) * double(phi);
-                storeResult(P, idx, P.G * mi * phi, P.G * gx, P.G * gy, P.G * gz);
-            }
-        }
-        pot = warpSum(pot);
-        if (lane == 0)
-        {
-            atomicAdd(&P.ctl->potential, pot);
-            if (P.sysPotential) atomicAdd(P.sysPotential + (P.groupSys ? P.groupSys[g] : 0u), pot);
-        }
+        const float phi = float(s[0]), mi = tgt.scalar(idx);
+        storeResult(P, idx, P.G * mi * phi, P.G * float(s[1]), P.G * float(s[2]), P.G * float(s[3]));
+        return double(mi) * double(phi);
     }
-    // every lane of a warp holds the same counts; one set of atomics per block
-    __shared__ unsigned long long sh[4][kFinishThreads / kWarp];
-    const int warp = threadIdx.x / kWarp;
-    if (lane == 0) sh[0][warp] = sumP, sh[1][warp] = sumM, sh[2][warp] = maxP, sh[3][warp] = maxM;
-    __syncthreads();
-    if (threadIdx.x != 0) return;
-    for (int k = 1; k < kFinishThreads / kWarp; ++k)
-    {
-        sumP += sh[0][k];
-        sumM += sh[1][k];
-        maxP = max(maxP, sh[2][k]);
-        maxM = max(maxM, sh[3][k]);
-    }
-    if (sumP == 0 && sumM == 0) return;
-    atomicAdd(&P.ctl->stats[kSumP2P], sumP);
-    atomicMax(&P.ctl->stats[kMaxP2P], maxP);
-    atomicAdd(&P.ctl->stats[kSumM2P], sumM);
-    atomicMax(&P.ctl->stats[kMaxM2P], maxM);
-}
+};
 
 template<class Nodes, class Targets, class Sources>
 static void launchTyped(const TraverseLaunch& t, const Nodes& nodes, const Targets& tgt, const Sources& src,
                         int smCount, cudaStream_t s)
 {
-    auto blocksFor = [&](auto kernel, size_t smem, size_t warps)
-    {
-        int perSm = 0;
-        RYO_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
-        RYO_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, kernel, kTravThreads, smem));
-        return unsigned(std::min((warps + kTravWarps - 1) / kTravWarps, size_t(std::max(perSm, 1)) * smCount));
-    };
     const size_t stack = sizeof(int) * kTravWarps * size_t(t.stackCapacity);
     if (t.subWalks == 0)
     {
         auto kernel       = traverseKernel<Nodes, Targets, Sources>;
         const size_t smem = stack + sizeof(WarpSmem) * kTravWarps;
-        kernel<<<blocksFor(kernel, smem, size_t(t.numGroups)), kTravThreads, smem, s>>>(t, nodes, tgt, src);
+        kernel<<<residentBlocks(kernel, smem, size_t(t.numGroups), smCount), kTravThreads, smem, s>>>(t, nodes, tgt, src);
         RYO_LAUNCH_CHECK();
         return;
     }
-    auto walk         = walkKernel<Nodes, Targets>;
-    auto eval         = evalKernel<Nodes, Targets, Sources>;
-    const size_t smem = stack + sizeof(WalkSmem) * kTravWarps;
-    walk<<<blocksFor(walk, smem, size_t(t.numGroups) * t.subWalks), kTravThreads, smem, s>>>(t, nodes, tgt);
+    launchWalk(t, nodes, tgt, smCount, s);
+    auto eval = evalKernel<Nodes, Targets, Sources>;
+    eval<<<residentBlocks(eval, 0, size_t(t.itemCapacity), smCount), kTravThreads, 0, s>>>(t, nodes, tgt, src);
     RYO_LAUNCH_CHECK();
-    eval<<<blocksFor(eval, 0, size_t(t.itemCapacity)), kTravThreads, 0, s>>>(t, nodes, tgt, src);
-    RYO_LAUNCH_CHECK();
-    const size_t fin = ceilDiv(size_t(t.numGroups) * kWarp, kFinishThreads);
-    finishKernel<<<unsigned(std::min(fin, size_t(8) * smCount)), kFinishThreads, 0, s>>>(t, tgt);
-    RYO_LAUNCH_CHECK();
+    launchFinish(t, FloatSink<Targets>{tgt}, smCount, s);
 }
 
 void launchTraverse(const TraverseLaunch& t, int smCount, cudaStream_t s)

@@ -15,8 +15,14 @@
  * counts equal the reference's. Evaluation stages 32 sources (one per lane) in shared memory as doubles and each
  * lane sums them for its two targets in FP64 registers; the FP64 pipe is half the FP32 rate on B200, and this path
  * trades that rate for the callers' precision.
+ *
+ * As in float, launches of few groups go through interaction lists (lists.cuh) and larger ones through the fused
+ * kernel. The list evaluation is bound by the FP64 pipe (13 operations, 26 cycles, per direct pair and sub-core) beside
+ * the conversions around rsqrt (24 cycles): it leaves the softening's maximum out where a batch lies beyond it. The step
+ * flow of 120,001 Plummer bodies, everything double: 2.3 ms per pass, against 6.3 ms with the fused kernel (whose time
+ * is its longest group's); 250,000 bodies of a cube, float masses: 2.48 against 2.75 ms.
  */
-#include "internal.hpp"
+#include "lists.cuh"
 
 namespace ryo
 {
@@ -203,6 +209,19 @@ __device__ void evalP2P64(WarpSmem64& S, int numLeaves, const Trav64<Th, Tm, Ta,
     }
 }
 
+//! adds a target's G m phi and G a to the outputs; returns m phi
+template<class Th, class Tm, class Ta, class Tmp>
+__device__ __forceinline__ double storeResult64(const TraverseLaunch& P, const Trav64<Th, Tm, Ta, Tmp>& A, int idx,
+                                                const Acc64& acc)
+{
+    const double mi = double(A.mt[idx]);
+    if (A.p) A.p[idx] += Ta(P.G64 * mi * acc.phi);
+    A.ax[idx] += Ta(P.G64 * acc.x);
+    A.ay[idx] += Ta(P.G64 * acc.y);
+    A.az[idx] += Ta(P.G64 * acc.z);
+    return mi * acc.phi;
+}
+
 template<bool kDipole, class Th, class Tm, class Ta, class Tmp>
 __global__ void __launch_bounds__(kT64Threads) traverseKernel64(TraverseLaunch P, Trav64<Th, Tm, Ta, Tmp> A)
 {
@@ -218,6 +237,7 @@ __global__ void __launch_bounds__(kT64Threads) traverseKernel64(TraverseLaunch P
         if (lane == 0) g = atomicAdd(&P.ctl->workCounter, 1u);
         g = __shfl_sync(0xffffffffu, g, 0);
         if (g >= unsigned(P.numGroups)) return;
+        if (P.groupList) g = P.groupList[g];
         const int b = int(P.groupStart[g]), e = int(P.groupEnd[g]);
 
         double px[2], py[2], pz[2];
@@ -366,15 +386,7 @@ __global__ void __launch_bounds__(kT64Threads) traverseKernel64(TraverseLaunch P
         for (int t = 0; t < 2; ++t)
         {
             int idx = b + t * kWarp + lane;
-            if (idx < e)
-            {
-                double mi = double(A.mt[idx]);
-                pot += mi * acc[t].phi;
-                if (A.p) A.p[idx] += Ta(P.G64 * mi * acc[t].phi);
-                A.ax[idx] += Ta(P.G64 * acc[t].x);
-                A.ay[idx] += Ta(P.G64 * acc[t].y);
-                A.az[idx] += Ta(P.G64 * acc[t].z);
-            }
+            if (idx < e) pot += storeResult64(P, A, idx, acc[t]);
         }
         pot = warpSum(pot);
         if (lane == 0)
@@ -392,6 +404,297 @@ __global__ void __launch_bounds__(kT64Threads) traverseKernel64(TraverseLaunch P
     }
 }
 
+// ------------------------------------------------------------------------------------------------ lists
+
+struct alignas(32) Center64
+{
+    double x, y, z, w; // centre and MAC r^2
+};
+
+__device__ __forceinline__ bool macFails(const Center64& c, const double tc[3], const double ts[3])
+{
+    const double v[4] = {c.x, c.y, c.z, c.w};
+    return macFails64(v, tc, ts);
+}
+
+//! the walk's view of the tree and of the targets
+struct Nodes64
+{
+    using Real   = double;
+    using Center = Center64;
+    const double* __restrict__ centers;
+    const int* __restrict__ childOffsets;
+    const int* __restrict__ internalToLeaf;
+    const uint32_t* __restrict__ layout;
+    __device__ __forceinline__ void load(int cell, Center64& c, int4& link) const
+    {
+        const double* cp = centers + 4 * size_t(cell);
+        c                = Center64{__ldg(cp), __ldg(cp + 1), __ldg(cp + 2), __ldg(cp + 3)};
+        link.x           = __ldg(childOffsets + cell);
+        if (link.x == 0)
+        {
+            const int leaf = __ldg(internalToLeaf + cell);
+            link.y         = int(__ldg(layout + leaf));
+            link.z         = int(__ldg(layout + leaf + 1)) - link.y;
+        }
+    }
+};
+struct Targets64
+{
+    const double* __restrict__ x;
+    const double* __restrict__ y;
+    const double* __restrict__ z;
+    __device__ __forceinline__ void position(int i, double p[3]) const
+    {
+        p[0] = __ldg(x + i), p[1] = __ldg(y + i), p[2] = __ldg(z + i);
+    }
+};
+
+struct EvalSmem64
+{
+    double stage[kWarp * kT64Stride];
+    int2 leaves[kWarp];
+    int leafScan[kWarp];
+};
+
+//! P2P of a pair beyond its softening
+__device__ __forceinline__ void p2p64far(Acc64& a, double tx, double ty, double tz, double sx, double sy, double sz,
+                                         double sm)
+{
+    double dx = sx - tx, dy = sy - ty, dz = sz - tz;
+    double r2 = dx * dx + dy * dy + dz * dz;
+    double ir = rsqrt64(r2);
+    double m3 = sm * ir * (ir * ir);
+    a.phi -= m3 * r2;
+    a.x += dx * m3;
+    a.y += dy * m3;
+    a.z += dz * m3;
+}
+
+/*! evaluates the interaction lists' items; their sums go to P.partials, or are the group's results when the item is its
+ *  only one */
+template<bool kDipole, class Th, class Tm, class Ta, class Tmp>
+__global__ void __launch_bounds__(kTravThreads, 4) evalKernel64(TraverseLaunch P, Trav64<Th, Tm, Ta, Tmp> A)
+{
+    constexpr int kVals = kDipole ? 12 : 8;
+    __shared__ EvalSmem64 smem[kTravWarps];
+    EvalSmem64& S  = smem[threadIdx.x / kWarp];
+    const int lane = laneId();
+    const unsigned numItems = min(P.ctl->itemCount, P.itemCapacity);
+    while (true)
+    {
+        unsigned it = 0;
+        if (lane == 0) it = atomicAdd(&P.ctl->itemHead, 1u);
+        it = __shfl_sync(0xffffffffu, it, 0);
+        if (it >= numItems) return;
+        const ListItem item = P.items[it];
+        const unsigned g    = item.group;
+        if (P.groupState[g] != 0u) continue;
+        const int b = int(P.groupStart[g]), e = int(P.groupEnd[g]);
+        const int idx[2] = {min(b + lane, e - 1), min(b + kWarp + lane, e - 1)};
+        double tx[2], ty[2], tz[2], lo[3], hi[3];
+        Th th[2];
+        // the targets where they are, or moved by a replica, and their bounds
+        auto place = [&](double sx, double sy, double sz)
+        {
+#pragma unroll
+            for (int t = 0; t < 2; ++t)
+            {
+                tx[t] = A.xt[idx[t]] + sx;
+                ty[t] = A.yt[idx[t]] + sy;
+                tz[t] = A.zt[idx[t]] + sz;
+            }
+            lo[0] = fmin(tx[0], tx[1]), hi[0] = fmax(tx[0], tx[1]);
+            lo[1] = fmin(ty[0], ty[1]), hi[1] = fmax(ty[0], ty[1]);
+            lo[2] = fmin(tz[0], tz[1]), hi[2] = fmax(tz[0], tz[1]);
+#pragma unroll
+            for (int o = kWarp / 2; o > 0; o >>= 1)
+#pragma unroll
+                for (int d = 0; d < 3; ++d)
+                {
+                    lo[d] = fmin(lo[d], __shfl_xor_sync(0xffffffffu, lo[d], o));
+                    hi[d] = fmax(hi[d], __shfl_xor_sync(0xffffffffu, hi[d], o));
+                }
+        };
+        place(0.0, 0.0, 0.0);
+        th[0] = A.ht[idx[0]], th[1] = A.ht[idx[1]];
+        Th hMax = th[0] < Th(0) ? -th[0] : th[0];
+        Th h1   = th[1] < Th(0) ? -th[1] : th[1];
+        hMax    = h1 > hMax ? h1 : hMax;
+        hMax    = warpMax(hMax);
+        Acc64 acc[2] = {{0, 0, 0, 0}, {0, 0, 0, 0}};
+        bool shifted = false;
+
+        const uint32_t* w = P.lists + size_t(it) * P.itemWords;
+        uint32_t pos = 0, hdr = 0, w0 = 0, w1 = 0;
+        auto fetch = [&](uint32_t at)
+        {
+            if (at < item.words) hdr = __ldg(w + at);
+            if (at + 1 + lane < item.words) w0 = __ldg(w + at + 1 + lane);
+            if (at + 1 + kWarp + lane < item.words) w1 = __ldg(w + at + 1 + kWarp + lane);
+        };
+        fetch(0);
+        while (pos < item.words)
+        {
+            const uint32_t kind = hdr & 3u;
+            const int n         = int(hdr >> 2);
+            const uint32_t c0 = w0, c1 = w1;
+            const uint32_t* payload = w + pos + 1;
+            pos += 1 + unsigned(kind == kSegLeaves || kind == kSegImages ? 2 * n : n);
+            fetch(pos);
+            __syncwarp();
+            if (kind == kSegReplica || (kind == kSegImages && shifted))
+            {
+                double sh[3] = {0.0, 0.0, 0.0};
+                shifted      = false;
+                if (kind == kSegReplica)
+                {
+#pragma unroll
+                    for (int d = 0; d < 3; ++d)
+                    {
+                        const int r = int(__shfl_sync(0xffffffffu, c0, d));
+                        shifted |= r != 0;
+                        sh[d] = r * P.boxL64[d];
+                    }
+                }
+                place(sh[0], sh[1], sh[2]);
+            }
+            if (kind == kSegCells || kind == kSegImages)
+            {
+                for (int k0 = 0; k0 < n; k0 += kWarp)
+                {
+                    const int count = min(kWarp, n - k0);
+                    if (lane < count)
+                    {
+                        const size_t cell = k0 == 0 ? c0 : c1;
+                        double* s         = S.stage + lane * kT64Stride;
+                        s[0]              = A.centers[4 * cell];
+                        s[1]              = A.centers[4 * cell + 1];
+                        s[2]              = A.centers[4 * cell + 2];
+                        if (kind == kSegImages)
+                        {
+                            // the image in the frame of the unshifted targets
+                            const uint32_t im = __ldg(payload + n + k0 + lane);
+#pragma unroll
+                            for (int d = 0; d < 3; ++d)
+                                s[d] -= double(imageShift(im, d)) * P.boxL64[d];
+                        }
+#pragma unroll
+                        for (int k = 0; k < kVals; ++k)
+                            s[3 + k] = double(A.multipoles[kVals * cell + k]);
+                    }
+                    __syncwarp();
+                    for (int j = 0; j < count; ++j)
+                    {
+                        const double* s = S.stage + j * kT64Stride;
+#pragma unroll
+                        for (int t = 0; t < 2; ++t)
+                            m2p64<kDipole>(acc[t], tx[t], ty[t], tz[t], s);
+                    }
+                    __syncwarp();
+                }
+            }
+            else if (kind == kSegLeaves)
+            {
+                int* to = reinterpret_cast<int*>(S.leaves);
+                if (lane < 2 * n) to[lane] = int(c0);
+                if (kWarp + lane < 2 * n) to[kWarp + lane] = int(c1);
+                __syncwarp();
+                const int2 mine = lane < n ? S.leaves[lane] : make_int2(0, 0);
+                const int inc   = warpInclusiveScan(mine.y);
+                S.leafScan[lane] = inc;
+                const int total = __shfl_sync(0xffffffffu, inc, kWarp - 1);
+                __syncwarp();
+                for (int r0 = 0; r0 < total; r0 += kWarp)
+                {
+                    const int r = r0 + lane;
+                    bool far    = true; // the staged body lies beyond every target's softening
+                    if (r < total)
+                    {
+                        int at = 0; // the first leaf whose inclusive prefix passes r
+#pragma unroll
+                        for (int o = kWarp / 2; o > 0; o >>= 1)
+                            if (S.leafScan[at + o - 1] <= r) at += o;
+                        const int2 lf  = S.leaves[at];
+                        const int body = lf.x + (r - (S.leafScan[at] - lf.y));
+                        const double x = A.xs[body], y = A.ys[body], z = A.zs[body];
+                        const Th h     = A.hs[body];
+                        double* s      = S.stage + lane * kT64Stride;
+                        *reinterpret_cast<double2*>(s)     = make_double2(x, y);
+                        *reinterpret_cast<double2*>(s + 2) = make_double2(z, double(A.ms[body]));
+                        reinterpret_cast<Th*>(s + 4)[0]    = h;
+                        const double dx = fmax(fmax(lo[0] - x, x - hi[0]), 0.0);
+                        const double dy = fmax(fmax(lo[1] - y, y - hi[1]), 0.0);
+                        const double dz = fmax(fmax(lo[2] - z, z - hi[2]), 0.0);
+                        const Th hij    = hMax + (h < Th(0) ? -h : h);
+                        // rounding aside; a pair this close to its softening takes the exact comparison
+                        far = dx * dx + dy * dy + dz * dz > 1.000001 * double(hij) * double(hij);
+                    }
+                    far = __all_sync(0xffffffffu, far);
+                    __syncwarp();
+                    const int n = min(kWarp, total - r0);
+                    if (far)
+                    {
+#pragma unroll 2
+                        for (int j = 0; j < n; ++j)
+                        {
+                            const double2 u = *reinterpret_cast<const double2*>(S.stage + j * kT64Stride);
+                            const double2 v = *reinterpret_cast<const double2*>(S.stage + j * kT64Stride + 2);
+#pragma unroll
+                            for (int t = 0; t < 2; ++t)
+                                p2p64far(acc[t], tx[t], ty[t], tz[t], u.x, u.y, v.x, v.y);
+                        }
+                    }
+                    else
+                    {
+                        for (int j = 0; j < n; ++j)
+                        {
+                            const double* s = S.stage + j * kT64Stride;
+                            const Th sh     = reinterpret_cast<const Th*>(s + 4)[0];
+#pragma unroll
+                            for (int t = 0; t < 2; ++t)
+                                p2p64(acc[t], tx[t], ty[t], tz[t], th[t], s[0], s[1], s[2], s[3], sh);
+                        }
+                    }
+                    __syncwarp();
+                }
+            }
+        }
+        if (!item.only)
+        {
+            double4* out = reinterpret_cast<double4*>(P.partials) + size_t(it) * (2 * kWarp);
+#pragma unroll
+            for (int t = 0; t < 2; ++t)
+                out[t * kWarp + lane] = make_double4(acc[t].phi, acc[t].x, acc[t].y, acc[t].z);
+            continue;
+        }
+        double pot = 0.0;
+#pragma unroll
+        for (int t = 0; t < 2; ++t)
+        {
+            const int i = b + t * kWarp + lane;
+            if (i < e) pot += storeResult64(P, A, i, acc[t]);
+        }
+        pot = warpSum(pot);
+        if (lane == 0) atomicAdd(&P.ctl->potential, pot);
+    }
+}
+
+//! finishKernel's sums and results
+template<class Th, class Tm, class Ta, class Tmp>
+struct DoubleSink
+{
+    Trav64<Th, Tm, Ta, Tmp> A;
+    __device__ __forceinline__ double4 part(const TraverseLaunch& P, size_t i) const
+    {
+        return reinterpret_cast<const double4*>(P.partials)[i];
+    }
+    __device__ __forceinline__ double store(const TraverseLaunch& P, int idx, const double s[4]) const
+    {
+        return storeResult64(P, A, idx, Acc64{s[0], s[1], s[2], s[3]});
+    }
+};
+
 template<class Th, class Tm, class Ta, class Tmp>
 static void launchTyped64(const TraverseLaunch& t, int smCount, cudaStream_t s)
 {
@@ -403,6 +706,16 @@ static void launchTyped64(const TraverseLaunch& t, int smCount, cudaStream_t s)
     A.multipoles = static_cast<const Tmp*>(t.multipoles64);
     A.p = static_cast<Ta*>(t.p64), A.ax = static_cast<Ta*>(t.ax64), A.ay = static_cast<Ta*>(t.ay64);
     A.az = static_cast<Ta*>(t.az64);
+    if (t.subWalks > 0)
+    {
+        launchWalk(t, Nodes64{t.centers64, t.childOffsets, t.internalToLeaf, t.layout},
+                   Targets64{t.xt64, t.yt64, t.zt64}, smCount, s);
+        auto eval = t.mdqArrays ? evalKernel64<true, Th, Tm, Ta, Tmp> : evalKernel64<false, Th, Tm, Ta, Tmp>;
+        eval<<<residentBlocks(eval, 0, size_t(t.itemCapacity), smCount), kTravThreads, 0, s>>>(t, A);
+        RYO_LAUNCH_CHECK();
+        launchFinish(t, DoubleSink<Th, Tm, Ta, Tmp>{A}, smCount, s);
+        return;
+    }
     auto kernel = t.mdqArrays ? traverseKernel64<true, Th, Tm, Ta, Tmp> : traverseKernel64<false, Th, Tm, Ta, Tmp>;
     size_t smem = sizeof(WarpSmem64) * kT64Warps + sizeof(int) * kT64Warps * size_t(t.stackCapacity);
     RYO_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));

@@ -120,3 +120,82 @@ def test_long_groups_of_a_large_solve():
     r = torch.stack([rx, ry, rz])
     err = ((a - r).norm(dim=0) / r.norm(dim=0)).cpu().numpy()
     assert np.percentile(err, 99) < 1e-3 and np.median(err) < 2e-4  # the expansions' error at theta 0.5
+
+
+def _double_rule(groups, x, y, z, m, h, tree, layout, centers, mp, shells, L):
+    """the traversal's rule and sums in numpy float64: per group (cells, bodies) and per body (-phi, ax, ay, az)"""
+    child, leaf = tree["childOffsets"], tree["internalToLeaf"]
+    pos, out, cells, bodies = np.stack([x, y, z], 1), np.zeros((len(x), 4)), [], []
+    for b, e in zip(groups[:-1], groups[1:]):
+        t = pos[b:e]
+        lo, hi = t.min(0), t.max(0)
+        tc, ts, nM, nP, acc = (hi + lo) * 0.5, (hi - lo) * 0.5, 0, 0, np.zeros((e - b, 4))
+        for k in np.ndindex(*(2 * shells + 1,) * 3):
+            sh = (np.array(k[::-1]) - shells) * L
+            tc = tc + sh
+            front, at = np.arange(1, 9), t + sh
+            while len(front):
+                d = np.maximum(np.abs(tc - centers[front, :3]) - ts, 0.0)
+                close = (d * d).sum(1) < centers[front, 3]
+                node = child[front] != 0
+                count = np.where(node, 1, layout[leaf[front] + 1] - layout[leaf[front]])
+                far = front[~close | (~node & (count == 0) & (centers[front, 3] != 0))]
+                nM += len(far)
+                for c in far:
+                    r = at - centers[c, :3]
+                    q, i1 = mp[c], 1 / np.sqrt((r * r).sum(1))
+                    Q = np.array([[q[1], q[2], q[3]], [q[2], q[4], q[5]], [q[3], q[5], q[6]]])
+                    Qr = r @ Q
+                    rQr = (r * Qr).sum(1)
+                    acc[:, 0] += q[0] * i1 + 0.5 * i1 ** 5 * rQr
+                    acc[:, 1:] += i1[:, None] ** 5 * Qr - ((2.5 * rQr * i1 ** 5 + q[0] * i1) * i1 * i1)[:, None] * r
+                for c in front[close & ~node & (count > 0)]:
+                    s = slice(layout[leaf[c]], layout[leaf[c] + 1])
+                    nP += s.stop - s.start
+                    d = pos[None, s] - at[:, None]
+                    r2 = (d * d).sum(2)
+                    w = m[None, s] / np.maximum(r2, (h[b:e, None] + h[None, s]) ** 2) ** 1.5
+                    acc[:, 0] += (w * r2).sum(1)
+                    acc[:, 1:] += (w[:, :, None] * d).sum(1)
+                front = (child[front[close & node]][:, None] + np.arange(8)).ravel()
+            tc = tc - sh
+        cells.append(nM)
+        bodies.append(nP)
+        out[b:e] = acc
+    return np.array(cells), np.array(bodies), out
+
+
+# a partial group, whole and ragged groups, softenings beyond and within the pairs' distances, replicas
+@pytest.mark.parametrize("kind", ["f64", "mixed"])
+@pytest.mark.parametrize("n,bucket,eps,shells", [(70, 8, 0.01, 0), (1000, 16, 1e-6, 0), (2051, 8, 0.2, 0),
+                                                 (640, 16, 0.01, 1)])
+def test_double_lists_against_numpy(kind, n, bucket, eps, shells):
+    import ryoanji_b200 as ryo
+    rng = np.random.default_rng(n)
+    real = torch.float64 if kind == "f64" else torch.float32
+    x, y, z = (dev(rng.uniform(-1, 1, n)) for _ in range(3))
+    tb, box = ryo.TreeBuilder(bucket), ryo.Box.cube(-1.0, 1.0)
+    nn = tb.update(x, y, z, box)
+    m, h = dev(rng.uniform(0.5, 1.5, n) / n).to(real), dev(rng.uniform(0.5, 1.5, n) * eps).to(real)
+    centers = torch.zeros(nn, 4, device="cuda", dtype=torch.float64)
+    mp = torch.zeros(nn, 8, device="cuda", dtype=real)
+    ryo.compute_leaf_source_center(x, y, z, m, tb.leafToInternal(), tb.layout(), centers)
+    ryo.upsweep_centers(tb.maxTreeLevel, tb.levelRange, tb.childOffsets(), centers)
+    ryo.compute_leaf_multipoles(x, y, z, m, tb.leafToInternal(), tb.layout(), centers, mp)
+    for level in range(tb.maxTreeLevel - 1, -1, -1):
+        ryo.upsweep_multipoles(tb.levelRange[level], tb.levelRange[level + 1], tb.childOffsets(), centers, mp)
+    ryo.set_mac(tb.nodeKeys(), centers, 2.0, box)
+    groups = ryo.compute_fixed_groups(0, n, 64)
+    out = [torch.zeros(n, device="cuda", dtype=real) for _ in range(4)]
+    pot, gm, gp = ryo.traverse(groups, 1, x, y, z, m, h, x, y, z, m, h, tb.childOffsets(), tb.internalToLeaf(),
+                               tb.layout(), centers, mp, 1.0, shells, box.lengths, *out, group_counts=True)
+    X, Y, Z, M, H, C, Q = (host(a).astype(np.float64) for a in (x, y, z, m, h, centers, mp))
+    tree = dict(childOffsets=host(tb.childOffsets()), internalToLeaf=host(tb.internalToLeaf()))
+    cells, bodies, acc = _double_rule(host(groups), X, Y, Z, M, H, tree, host(tb.layout()), C, Q, shells, 2.0)
+    assert np.array_equal(host(gm), cells) and np.array_equal(host(gp), bodies)
+    # the single-precision rsqrt enters every term with up to 2 ulp, five times in a quadrupole's
+    scale = np.maximum(np.linalg.norm(acc[:, 1:], axis=1), 0.25 * (1 + 26 * shells))
+    err = np.linalg.norm(np.stack([host(a) for a in out[1:]], 1) - acc[:, 1:], axis=1) / scale
+    assert err.max() < 3e-6
+    assert np.allclose(host(out[0]), -M * acc[:, 0], rtol=2e-6)
+    assert pot == pytest.approx(-0.5 * float((M * acc[:, 0]).sum()), rel=2e-6)
