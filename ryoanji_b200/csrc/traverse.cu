@@ -34,6 +34,7 @@
  *   - the MAC test uses explicitly rounded single operations so that every decision is reproducible bit for bit.
  */
 #include "lists.cuh"
+#include "packed.cuh"
 
 namespace ryo
 {
@@ -67,56 +68,6 @@ static_assert(2 * kWarp - 1 + kWarp <= kM2PCap + kWarp, "the pending cell list m
 // a P2P evaluation leaves fewer than kP2PBatch bodies, so at most kP2PBatch - 1 leaves, pending; one walk step adds
 // at most kWarp more
 static_assert(kP2PBatch - 1 + kWarp <= kLeafCap + kWarp, "the pending leaf list must hold a step's additions");
-
-// ------------------------------------------------------------------------------------------------ packed f32x2
-
-using f2 = unsigned long long; // two floats: low half target 0, high half target 1
-
-__device__ __forceinline__ f2 pk(float lo, float hi)
-{
-    f2 r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-    return r;
-}
-__device__ __forceinline__ void upk(f2 v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
-__device__ __forceinline__ f2 add2(f2 a, f2 b)
-{
-    f2 r;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ f2 sub2(f2 a, f2 b)
-{
-    f2 r;
-    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ f2 mul2(f2 a, f2 b)
-{
-    f2 r;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c)
-{
-    f2 r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
-
-__device__ __forceinline__ float rsqrtApprox(float x)
-{
-    float y;
-    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
-
-__device__ __forceinline__ f2 rsqrt2(f2 v)
-{
-    float a, b;
-    upk(v, a, b);
-    return pk(rsqrtApprox(a), rsqrtApprox(b));
-}
 
 //! packed accumulators of a lane's two targets: P = -phi, X, Y, Z = acceleration
 struct Acc2
