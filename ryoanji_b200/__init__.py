@@ -493,7 +493,7 @@ class TreeBuilder:
         return nn.value
 
     def _wrap(self, ptr, count, dtype):
-        return _abi.wrap_device(ptr, count, dtype, self._device)
+        return _abi.wrap_device(ptr, count, dtype, self._device, self)
 
     @property
     def numLeafNodes(self) -> int:
@@ -846,7 +846,7 @@ def solve_arrays(ctx: Context | None = None, device=None) -> dict:
     _check(lib.ryo_solve_arrays_get(ctx.handle, C.byref(a)), ctx)
     dev = device or torch.device("cuda", ctx.device)
     nl, nn, ng = a.numLeaves, a.numNodes, a.numGroups
-    w = lambda ptr, cnt, dt: _abi.wrap_device(ptr, cnt, dt, dev)  # noqa: E731
+    w = lambda ptr, cnt, dt: _abi.wrap_device(ptr, cnt, dt, dev, ctx)  # noqa: E731
     nd = w(a.nodeData, 16 * nn, torch.float32).view(nn, 16)
     return dict(numLeafNodes=nl, numNodes=nn, numGroups=ng, leaves=w(a.leaves, nl + 1, torch.int64),
                 layout=w(a.layout, nl + 1, torch.int32), prefixes=w(a.prefixes, nn, torch.int64),

@@ -248,7 +248,8 @@ lib = _LazyLib()
 
 
 class _CudaArray:
-    def __init__(self, ptr: int, count: int, typestr: str):
+    def __init__(self, ptr: int, count: int, typestr: str, owner):
+        self.owner = owner  # a tensor keeps its _CudaArray, and with it the memory's owner
         self.__cuda_array_interface__ = {"shape": (count,), "typestr": typestr, "data": (int(ptr), False),
                                          "version": 3, "strides": None}
 
@@ -256,8 +257,9 @@ class _CudaArray:
 _TYPESTR = {torch.int32: "<i4", torch.int64: "<i8", torch.float32: "<f4", torch.float64: "<f8"}
 
 
-def wrap_device(ptr, count: int, dtype, device) -> torch.Tensor:
-    """a torch view of library-owned device memory (valid until the owner reallocates it)"""
+def wrap_device(ptr, count: int, dtype, device, owner) -> torch.Tensor:
+    """a torch view of device memory of @p owner, which lives as long as the view (valid until the owner reallocates
+    it)"""
     if not ptr or count == 0:
         return torch.empty(0, dtype=dtype, device=device)
-    return torch.as_tensor(_CudaArray(ptr, count, _TYPESTR[dtype]), device=device)
+    return torch.as_tensor(_CudaArray(ptr, count, _TYPESTR[dtype], owner), device=device)
