@@ -5,9 +5,13 @@
  * traversal covers the (2 numReplicaShells + 1)^3 replica boxes; the correction adds, per target, the real-space
  * images of the root multipole with erfc weights (-erf inside the replicated region) and the reciprocal-space sum.
  *
- * B200 form: one warp per target group, lanes over its targets. Real space runs in float. The reciprocal sum runs in
- * double: per target the three phase factors exp(2 pi i dx_d / L) are computed once and every wave vector's
- * exp(i k.r) is a product of their integer powers, so no trigonometric call is made per wave vector.
+ * B200 form: two warps per target group, lanes over its targets. Real space runs in float; columns of images that lie
+ * beyond the cutoff as a whole are passed over. The reciprocal sum runs in double: per target the three phase factors
+ * exp(2 pi i dx_d / L) are computed once and every wave vector's exp(i k.r) is a product of their integer powers, so no
+ * trigonometric call is made per wave vector. The wave vectors k and -k add the same cosine term to the potential and
+ * the same sine term to the force, and their terms odd in k cancel, so one of each pair is summed with twice its
+ * coefficient. Bound by instruction issue (erfc and exp of the images). 2^18 bodies, against one warp per group, every
+ * image and every wave vector: a solve takes 75 us less, 1.935 -> 1.860 ms.
  */
 #include <cmath>
 
@@ -25,11 +29,11 @@ struct EwaldKernelParams
     double centerD[3];
     R L, lCut2, alpha, alpha2, k1, ka, smallR2;
     int replicaShells, ewaldShells;
-    int numK;
+    int numK; // pairs (k, -k), in runs of one (kx, ky)
     double twoPiOverL;
-    signed char h[kEwaldMaxK][3];
-    double fc[kEwaldMaxK];
-    double fs[kEwaldMaxK];
+    signed char h[kEwaldMaxK / 2][3];
+    double hd[kEwaldMaxK / 2][3];
+    double fc2[kEwaldMaxK / 2]; // twice the cosine coefficient
 };
 
 //! ewaldEvalMultipoleComplete (ewald.hpp:90-115)
@@ -115,7 +119,7 @@ __device__ inline double rsErf(double v) { return erf(v); }
 __device__ inline float rsErfc(float v) { return erfcf(v); }
 __device__ inline double rsErfc(double v) { return erfc(v); }
 
-/*! one warp per target group. R is the real-space type: float for the reference's float instantiation, double for its
+/*! two warps per target group. R is the real-space type: float for the reference's float instantiation, double for its
  *  double-coordinate ones (ryoanji/src/ryoanji/interface/ewald.cu:101-110), where the reference's real space runs in
  *  its coordinate type; the reciprocal sum is double in every set. Tc, Tm, Ta: coordinates, masses, outputs. */
 template<class R, class Tc, class Tm, class Ta>
@@ -124,13 +128,13 @@ __global__ void ewaldKernel(const __grid_constant__ EwaldKernelParams<R> E, cons
                             const Tc* __restrict__ y, const Tc* __restrict__ z, const Tm* __restrict__ m, float G,
                             Ta* ugrav, Ta* ax, Ta* ay, Ta* az, double* potential)
 {
-    int warpGlobal = (blockIdx.x * blockDim.x + threadIdx.x) / kWarp;
-    int lane       = laneId();
-    double upot    = 0.0;
-    if (warpGlobal < int(numGroups))
+    const unsigned warpGlobal = (blockIdx.x * blockDim.x + threadIdx.x) / kWarp;
+    const int lane            = laneId();
+    double upot               = 0.0;
+    if (warpGlobal / 2 < numGroups)
     {
-        uint32_t b = groupStart[warpGlobal], e = groupEnd[warpGlobal];
-        for (uint32_t i = b + lane; i < e; i += kWarp)
+        uint32_t b = groupStart[warpGlobal / 2], e = groupEnd[warpGlobal / 2];
+        for (uint32_t i = b + (warpGlobal & 1) * kWarp + lane; i < e; i += 2 * kWarp)
         {
             R pos[3]  = {R(x[i]), R(y[i]), R(z[i])};
             R acc[4]  = {E.k1 * E.mroot[0], R(0), R(0), R(0)};
@@ -139,9 +143,14 @@ __global__ void ewaldKernel(const __grid_constant__ EwaldKernelParams<R> E, cons
             // real space (ewald.hpp:200-301)
             for (int ix = -S; ix <= S; ++ix)
                 for (int iy = -S; iy <= S; ++iy)
+                {
+                    // the column's smallest distance: the images' own operations, each monotonic
+                    const bool preXY = (-Rs <= ix && ix <= Rs) && (-Rs <= iy && iy <= Rs);
+                    const R cx = r[0] + ix * E.L, cy = r[1] + iy * E.L;
+                    if (cx * cx + cy * cy > E.lCut2 && !preXY) continue;
                     for (int iz = -S; iz <= S; ++iz)
                     {
-                        bool pre = (-Rs <= ix && ix <= Rs) && (-Rs <= iy && iy <= Rs) && (-Rs <= iz && iz <= Rs);
+                        bool pre = preXY && (-Rs <= iz && iz <= Rs);
                         R Rv[3]  = {r[0] + ix * E.L, r[1] + iy * E.L, r[2] + iz * E.L};
                         R R2     = Rv[0] * Rv[0] + (Rv[1] * Rv[1] + Rv[2] * Rv[2]);
                         if (R2 > E.lCut2 && !pre) continue;
@@ -180,6 +189,7 @@ __global__ void ewaldKernel(const __grid_constant__ EwaldKernelParams<R> E, cons
                         }
                         ewaldEval<R>(acc, Rv, g, E.mroot);
                     }
+                }
             // reciprocal space (ewald.hpp:303-327), double, exp(i k.r) from powers of the per-axis phases
             double dr[3] = {double(pos[0]) - E.centerD[0], double(pos[1]) - E.centerD[1],
                             double(pos[2]) - E.centerD[2]};
@@ -199,18 +209,21 @@ __global__ void ewaldKernel(const __grid_constant__ EwaldKernelParams<R> E, cons
                 pw[d][0]   = cmul(pw[d][1], e1c);
             }
             double kp = 0.0, ka3[3] = {0.0, 0.0, 0.0};
+            double2 xy = make_double2(0.0, 0.0); // exp(i (kx x + ky y)) of the current run
             for (int q = 0; q < E.numK; ++q)
             {
-                int hx = E.h[q][0], hy = E.h[q][1], hz = E.h[q][2];
-                double2 w = cmul(cmul(pw[0][hx + 3], pw[1][hy + 3]), pw[2][hz + 3]);
-                double c = w.x, s = w.y;
-                double sum  = E.fc[q] * c + E.fs[q] * s;
-                double diff = E.fc[q] * s - E.fs[q] * c;
-                kp -= sum;
-                ka3[0] += diff * (E.twoPiOverL * hx);
-                ka3[1] += diff * (E.twoPiOverL * hy);
-                ka3[2] += diff * (E.twoPiOverL * hz);
+                const int hx = E.h[q][0], hy = E.h[q][1], hz = E.h[q][2];
+                if (q == 0 || hx != E.h[q - 1][0] || hy != E.h[q - 1][1]) xy = cmul(pw[0][hx + 3], pw[1][hy + 3]);
+                const double2 w = cmul(xy, pw[2][hz + 3]);
+                const double t  = E.fc2[q] * w.y;
+                kp -= E.fc2[q] * w.x;
+                ka3[0] += t * E.hd[q][0];
+                ka3[1] += t * E.hd[q][1];
+                ka3[2] += t * E.hd[q][2];
             }
+#pragma unroll
+            for (int d = 0; d < 3; ++d)
+                ka3[d] *= E.twoPiOverL;
             double phi = double(acc[0]) + kp;
             double mi  = m[i];
             upot += phi * mi;
@@ -248,17 +261,22 @@ static void launchEwaldTyped(const EwaldHost& h, const uint32_t* groupStart, con
     E.smallR2       = R(h.smallR * h.L * h.L);
     E.replicaShells = h.replicaShells;
     E.ewaldShells   = h.ewaldShells;
-    E.numK          = h.numK;
+    E.numK          = 0;
     E.twoPiOverL    = 2 * M_PI / h.L;
     for (int q = 0; q < h.numK; ++q)
     {
+        // the half space of vectors whose first non-zero component is positive; the setup visits them by kx, ky, kz
+        const double* k = h.kdata + 5 * q;
+        if (!(k[0] > 0 || (k[0] == 0 && (k[1] > 0 || (k[1] == 0 && k[2] > 0))))) continue;
         for (int d = 0; d < 3; ++d)
-            E.h[q][d] = (signed char)h.kdata[5 * q + d];
-        E.fc[q] = h.kdata[5 * q + 3];
-        E.fs[q] = h.kdata[5 * q + 4];
+        {
+            E.h[E.numK][d]  = (signed char)k[d];
+            E.hd[E.numK][d] = k[d];
+        }
+        E.fc2[E.numK++] = 2 * k[3];
     }
     unsigned threads = 128;
-    unsigned blocks  = ceilDiv(size_t(numGroups) * kWarp, threads);
+    unsigned blocks  = ceilDiv(size_t(numGroups) * 2 * kWarp, threads);
     ewaldKernel<R, Tc, Tm, Ta><<<blocks, threads, 0, s>>>(E, groupStart, groupEnd, numGroups, x, y, z, m, G, ugrav,
                                                            ax, ay, az, potentialOut);
     RYO_LAUNCH_CHECK();
