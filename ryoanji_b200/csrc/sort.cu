@@ -7,9 +7,12 @@
  * with decoupled look-back (bounded waits), stage the tile in shared memory in digit order and write coalesced runs.
  * The sort is stable (keys and payload indices keep their input order within equal keys), as the reference needs.
  */
+#include <cooperative_groups.h>
 #include <mutex>
 
 #include "internal.hpp"
+
+namespace cg = cooperative_groups;
 
 namespace ryo
 {
@@ -390,11 +393,187 @@ __global__ void __launch_bounds__(kSortBlock, 4) onesweepPass(const uint64_t* __
     }
 }
 
+// ------------------------------------------------------------------------------------------------ cluster sort
+
+constexpr int kClusterThreads  = 1024;
+constexpr int kClusterWarps    = kClusterThreads / kWarp;
+constexpr int kClusterMaxItems = 2; // keys per thread
+constexpr int kClusterMaxCtas  = 8; // the portable cluster size
+constexpr size_t kClusterKeys  = size_t(kClusterThreads) * kClusterMaxItems * kClusterMaxCtas;
+
+constexpr size_t clusterSortBytes(int items)
+{
+    return size_t(kClusterThreads) * items * (sizeof(uint64_t) + sizeof(uint32_t)) +
+           kClusterWarps * kDigits * sizeof(uint32_t);
+}
+
+/*! the whole sort of up to kClusterKeys pairs by one cluster of blocks, in place: the pairs stay in registers and
+ *  change places through the cluster's shared memory once per digit. Bound by latency (ballots, barriers and remote
+ *  stores, about 4 us per digit), where the onesweep passes of so few keys are bound by their launches (8 us): a sort
+ *  call of 4,096 keys 111 -> 64 us, of 16,384 keys 120 -> 89 us. With four and eight keys per thread it was no faster
+ *  than the passes (24,000 keys 115 against 125 us, 65,536 keys 180 against 123 us), so it ends at two.
+ *  A padding item past n has all bits set; it starts behind every key and stays there, since the passes are stable. */
+template<int kItems>
+__global__ void __launch_bounds__(kClusterThreads) clusterSort(uint64_t* keys, uint32_t* vals, uint32_t n, int beginBit,
+                                                               int endBit, bool iotaValues)
+{
+    constexpr uint32_t kBlockKeys = kClusterThreads * kItems;
+    extern __shared__ __align__(16) unsigned char smem[];
+    uint64_t* sKeys           = reinterpret_cast<uint64_t*>(smem);
+    uint32_t* sVals           = reinterpret_cast<uint32_t*>(sKeys + kBlockKeys);
+    uint32_t(*sHist)[kDigits] = reinterpret_cast<uint32_t(*)[kDigits]>(sVals + kBlockKeys);
+    __shared__ uint32_t sQuarter[4][kDigits];
+    __shared__ uint32_t sTotal[kDigits];
+    __shared__ uint32_t sWarp[32];
+    cg::cluster_group cl = cg::this_cluster();
+    const unsigned rank = cl.block_rank(), ctas = cl.num_blocks();
+    const int tid = threadIdx.x, lane = laneId(), warp = tid / kWarp;
+    const int digit = tid & (kDigits - 1), quarter = tid / kDigits;
+    const unsigned lt    = lanemaskLt();
+    const uint32_t local = uint32_t(warp) * (kItems * kWarp) + lane;
+    const uint32_t first = rank * kBlockKeys + local;
+    uint64_t k[kItems];
+    uint32_t v[kItems], r[kItems];
+#pragma unroll
+    for (int i = 0; i < kItems; ++i)
+    {
+        const uint32_t at = first + i * kWarp;
+        k[i]              = at < n ? keys[at] : ~uint64_t(0);
+        v[i]              = at < n ? (iotaValues ? at : vals[at]) : 0u;
+    }
+    for (int shift = beginBit; shift < endBit; shift += 8)
+    {
+        const int nbits      = min(8, endBit - shift);
+        const uint32_t dmask = (1u << nbits) - 1;
+        for (int i = tid; i < kClusterWarps * kDigits; i += kClusterThreads)
+            (&sHist[0][0])[i] = 0;
+        __syncthreads();
+        // rank within the warp, in input order: as onesweepPass
+#pragma unroll
+        for (int i = 0; i < kItems; ++i)
+        {
+            const uint32_t d = uint32_t(k[i] >> shift) & dmask;
+            unsigned peers   = 0xffffffffu;
+#pragma unroll
+            for (int b = 0; b < 8; ++b)
+            {
+                if (b >= nbits) break;
+                const bool bit    = (d >> b) & 1u;
+                const unsigned bv = __ballot_sync(0xffffffffu, bit);
+                peers &= bit ? bv : ~bv;
+            }
+            const int leader = __ffs(peers) - 1;
+            uint32_t before  = 0;
+            if (lane == leader)
+            {
+                before         = sHist[warp][d];
+                sHist[warp][d] = before + __popc(peers);
+            }
+            before = __shfl_sync(0xffffffffu, before, leader);
+            r[i]   = before + __popc(peers & lt);
+        }
+        __syncthreads();
+        // thread (digit, quarter): the digit's offsets over a quarter of the warps, then over the quarters
+        uint32_t sum = 0;
+#pragma unroll
+        for (int w = 0; w < kClusterWarps / 4; ++w)
+        {
+            uint32_t& slot   = sHist[quarter * (kClusterWarps / 4) + w][digit];
+            const uint32_t c = slot;
+            slot             = sum;
+            sum += c;
+        }
+        sQuarter[quarter][digit] = sum;
+        __syncthreads();
+        uint32_t mine = 0, total = 0;
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+        {
+            const uint32_t c = sQuarter[q][digit];
+            mine += q < quarter ? c : 0u;
+            total += c;
+        }
+        if (quarter == 0) sTotal[digit] = total;
+        // the counts are out, and no block reads the pairs of the digit before any more
+        cl.sync();
+        uint32_t all = 0;
+        for (unsigned c = 0; c < ctas; ++c)
+        {
+            const uint32_t t = *cl.map_shared_rank(&sTotal[digit], c);
+            mine += c < rank ? t : 0u;
+            all += t;
+        }
+        const uint32_t incl = blockInclusiveScan(quarter == 0 ? all : 0u, sWarp, (uint32_t*)nullptr);
+        if (quarter == 0) sQuarter[0][digit] = incl - all;
+        __syncthreads();
+        mine += sQuarter[0][digit];
+#pragma unroll
+        for (int w = 0; w < kClusterWarps / 4; ++w)
+            sHist[quarter * (kClusterWarps / 4) + w][digit] += mine;
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < kItems; ++i)
+        {
+            const uint32_t at  = sHist[warp][uint32_t(k[i] >> shift) & dmask] + r[i];
+            const unsigned dst = at / kBlockKeys, slot = at % kBlockKeys;
+            *cl.map_shared_rank(sKeys + slot, dst) = k[i];
+            *cl.map_shared_rank(sVals + slot, dst) = v[i];
+        }
+        cl.sync();
+#pragma unroll
+        for (int i = 0; i < kItems; ++i)
+        {
+            k[i] = sKeys[local + i * kWarp];
+            v[i] = sVals[local + i * kWarp];
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < kItems; ++i)
+    {
+        const uint32_t at = first + i * kWarp;
+        if (at < n)
+        {
+            keys[at] = k[i];
+            vals[at] = v[i];
+        }
+    }
+}
+
+template<int kItems>
+static void launchClusterSort(uint64_t* keys, uint32_t* vals, size_t n, int beginBit, int endBit, bool iotaValues,
+                              cudaStream_t s)
+{
+    constexpr size_t kBlockKeys = size_t(kClusterThreads) * kItems;
+    RYO_CUDA(cudaFuncSetAttribute(clusterSort<kItems>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  int(clusterSortBytes(kItems))));
+    cudaLaunchAttribute attr;
+    attr.id               = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = unsigned((n + kBlockKeys - 1) / kBlockKeys);
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim          = dim3(attr.val.clusterDim.x);
+    cfg.blockDim         = dim3(kClusterThreads);
+    cfg.dynamicSmemBytes = clusterSortBytes(kItems);
+    cfg.stream           = s;
+    cfg.attrs            = &attr;
+    cfg.numAttrs         = 1;
+    RYO_CUDA(cudaLaunchKernelEx(&cfg, clusterSort<kItems>, keys, vals, uint32_t(n), beginBit, endBit, iotaValues));
+    RYO_LAUNCH_CHECK();
+}
+
 bool radixSortPairs(uint64_t* keys, uint32_t* values, uint64_t* keysAlt, uint32_t* valuesAlt, size_t n, int beginBit,
                     int endBit, void* tmp, size_t tmpBytes, unsigned int* errorFlag, cudaStream_t s, bool iotaValues)
 {
     if (n == 0) return false;
     if (tmpBytes < sortTempBytes(n)) throw CudaError{cudaErrorInvalidValue, "radix sort: temporary storage too small"};
+    if (n <= kClusterKeys)
+    {
+        // one launch instead of two clears and a launch per digit; the fewest keys per thread that the cluster allows
+        const size_t items = (n + kClusterThreads * kClusterMaxCtas - 1) / (kClusterThreads * kClusterMaxCtas);
+        if (items <= 1) launchClusterSort<1>(keys, values, n, beginBit, endBit, iotaValues, s);
+        else launchClusterSort<2>(keys, values, n, beginBit, endBit, iotaValues, s);
+        return false;
+    }
     int numPasses = (endBit - beginBit + 7) / 8;
     SortTemp t    = sortLayout(tmp, n);
     RYO_CUDA(cudaMemsetAsync(tmp, 0, t.headBytes, s));
