@@ -175,9 +175,12 @@ extern "C" ryo_status ryo_ctx_create(int device, ryo_ctx_t** out)
                                 RYO_CUDA(cudaDeviceGetAttribute(&ctx->smCount, cudaDevAttrMultiProcessorCount, device));
                                 RYO_CUDA(cudaMalloc(&ctx->ctl, sizeof(Control)));
                                 RYO_CUDA(cudaMemset(ctx->ctl, 0, sizeof(Control)));
+                                RYO_CUDA(cudaHostAlloc(&ctx->results, sizeof(HostResults), cudaHostAllocDefault));
                             });
     if (st != RYO_OK)
     {
+        ctx->releaseAll();
+        if (ctx->ctl) cudaFree(ctx->ctl);
         delete ctx;
         return st;
     }
@@ -591,6 +594,14 @@ void checkCallerGroups(const ryo_group_view* grp, cudaStream_t stream)
                 "traverse: every group needs 1 to 64 targets within [firstBody, lastBody)");
 }
 
+//! the control block after the work queued on @p s, for which this waits
+void readControl(ryo_ctx* ctx, Control& c, cudaStream_t s)
+{
+    RYO_CUDA(cudaMemcpyAsync(&ctx->results->ctl, ctx->ctl, sizeof(Control), cudaMemcpyDeviceToHost, s));
+    RYO_CUDA(cudaStreamSynchronize(s));
+    c = ctx->results->ctl;
+}
+
 /*! traverses t's groups, or those of @p list, through interaction lists until every group has been served or has
  *  overflowed the stack. Lists are cut by the solve's group count and the walk alone, so a group's sums do not depend
  *  on the launch or pass that it falls in. */
@@ -627,8 +638,7 @@ void traverseLists(ryo_ctx* ctx, TraverseLaunch t, const uint32_t* list, uint32_
             t.numGroups      = int(std::min(chunk, count - first));
             t.unservedGroups = unserved[flip] + left;
             launchTraverse(t, ctx->smCount, s);
-            RYO_CUDA(cudaMemcpyAsync(&c, ctx->ctl, sizeof(Control), cudaMemcpyDeviceToHost, s));
-            RYO_CUDA(cudaStreamSynchronize(s));
+            readControl(ctx, c, s);
             left += c.unservedCount;
             if (left > 0 || first + chunk < count) launchTraversalReset(ctx->ctl, kTravLists, s);
         }
@@ -672,8 +682,7 @@ void runTraversal(ryo_ctx* ctx, TraverseLaunch t, cudaStream_t s, double* potent
             t.heavyCapacity = uint32_t(t.numGroups);
             t.heavyCost     = kHeavyCost;
             launchTraverse(t, ctx->smCount, s);
-            RYO_CUDA(cudaMemcpyAsync(&hc, ctx->ctl, sizeof(Control), cudaMemcpyDeviceToHost, s));
-            RYO_CUDA(cudaStreamSynchronize(s));
+            readControl(ctx, hc, s);
             if (hc.heavyCount > 0)
             {
                 // groups too long for one warp go through lists, whose pieces all warps share
@@ -725,7 +734,11 @@ void runTraversal(ryo_ctx* ctx, TraverseLaunch t, cudaStream_t s, double* potent
         ctx->hostStats[i] = hc.stats[i];
     if (unsplittable) ctx->hostStats[kMaxP2P] = 0xFFFFFFFFull;
     if (potentialOut) *potentialOut = hc.potential;
-    if (hc.error) throw ApiError{RYO_ERR_TIMEOUT, "traversal: a device-side bounded wait timed out"};
+    if (hc.error)
+    {
+        RYO_CUDA(cudaMemsetAsync(&ctx->ctl->error, 0, sizeof(unsigned int), s));
+        throw ApiError{RYO_ERR_TIMEOUT, "traversal: a device-side bounded wait timed out"};
+    }
 }
 
 } // namespace
@@ -1128,9 +1141,10 @@ void treebuilderUpdate(ryo_treebuilder* tb, T* x, T* y, T* z, size_t n, const De
     tb->oct.internalToLeaf = tb->buf<int>(".internalToLeaf", nn, s);
     tb->oct.leafToInternal = tb->buf<int>(".leafToInternal", nn, s);
     tb->oct.d_levelRange   = tb->buf<int>(".levelRange", kMaxLevel + 2, s);
-    linkOctree(ctx, tb->leaves, nl, tb->oct, tb->levelRange, s);
+    linkOctree(ctx, tb->leaves, nl, tb->oct, nullptr, s);
     tb->numBodies = n;
     checkDeviceError(ctx, s);
+    std::copy(ctx->results->levelRange, ctx->results->levelRange + kMaxLevel + 2, tb->levelRange);
 }
 } // namespace
 
@@ -1325,8 +1339,8 @@ void solveSingle(ryo_ctx* ctx, const ryo_solve_params* P, float* x, float* y, fl
     {
         double* mm = ctx->scratch<double>("solve.bbox", 6, s);
         launchBoundingBox(x, y, z, n, mm, s);
-        double hb[6];
-        RYO_CUDA(cudaMemcpyAsync(hb, mm, sizeof(hb), cudaMemcpyDeviceToHost, s));
+        double* hb = ctx->results->bbox;
+        RYO_CUDA(cudaMemcpyAsync(hb, mm, 6 * sizeof(double), cudaMemcpyDeviceToHost, s));
         RYO_CUDA(cudaStreamSynchronize(s));
         double ext = std::max({hb[1] - hb[0], hb[3] - hb[2], hb[5] - hb[4]});
         if (!(ext > 0)) ext = 1.0;
@@ -1417,8 +1431,9 @@ void solveSingle(ryo_ctx* ctx, const ryo_solve_params* P, float* x, float* y, fl
     oct.internalToLeaf = ctx->scratch<int>("solve.internalToLeaf", nn, s);
     oct.leafToInternal = ctx->scratch<int>("solve.leafToInternal", nn, s);
     oct.d_levelRange   = ctx->scratch<int>("solve.levelRange", kMaxLevel + 2, s);
+    // the level ranges are needed here only for large trees; otherwise they arrive by the traversal's end
     int levelRange[kMaxLevel + 2];
-    linkOctree(ctx, leaves, nl, oct, levelRange, s);
+    linkOctree(ctx, leaves, nl, oct, nn >= kLevelUpsweepNodes ? levelRange : nullptr, s);
     if (pipe) permute();
 
     mark(ctx, P, 2, s);
@@ -1433,6 +1448,7 @@ void solveSingle(ryo_ctx* ctx, const ryo_solve_params* P, float* x, float* y, fl
     launchFusedUpsweep(ctx, xyzm, nl, nn, layout, oct.leafToInternal + ni, oct.childOffsets,
                        oct.parents, oct.prefixes, 1.0f / P->theta, dbox, records, nullptr, nullptr,
                        root, s, nullptr, 0, nullptr, dipoles, 0, levelRange);
+    RYO_CUDA(cudaMemcpyAsync(ctx->results->root, root, sizeof(double) * 11, cudaMemcpyDeviceToHost, s));
 
     mark(ctx, P, 3, s);
     // groups and traversal
@@ -1461,9 +1477,6 @@ void solveSingle(ryo_ctx* ctx, const ryo_solve_params* P, float* x, float* y, fl
     // straight into them: the results cross the link while the traversal runs, and no download follows it
     float* mapped[4]  = {nullptr, nullptr, nullptr, nullptr};
     const bool direct = pipe && !periodic && mappedHostOutputs(pipe, n, mapped);
-    if (!direct)
-        for (float* a : {p, ax, ay, az})
-            RYO_CUDA(cudaMemsetAsync(a, 0, n * sizeof(float), s));
     TraverseLaunch t{};
     t.groupStart    = groups;
     t.groupEnd      = groups + 1;
@@ -1483,15 +1496,14 @@ void solveSingle(ryo_ctx* ctx, const ryo_solve_params* P, float* x, float* y, fl
     t.ax = direct ? mapped[1] : ax;
     t.ay = direct ? mapped[2] : ay;
     t.az = direct ? mapped[3] : az;
-    t.overwrite     = direct ? 1 : 0;
+    t.overwrite     = 1; // every body is in one group
     t.stackCapacity = P->stackCapacity;
     t.dipoles       = dipoles;
     t.softeningRange = hRange;
     t.massRange      = dipoles ? nullptr : hRange + 2; // signed-mass expansions keep the per-source mass
-    uint32_t* gm2p  = ctx->scratch<uint32_t>("solve.groupM2P", numGroups, s);
-    uint32_t* gp2p  = ctx->scratch<uint32_t>("solve.groupP2P", numGroups, s);
-    RYO_CUDA(cudaMemsetAsync(gm2p, 0, sizeof(uint32_t) * numGroups, s));
-    RYO_CUDA(cudaMemsetAsync(gp2p, 0, sizeof(uint32_t) * numGroups, s));
+    uint32_t* gm2p  = ctx->scratch<uint32_t>("solve.groupCounts", 2 * size_t(numGroups), s);
+    uint32_t* gp2p  = gm2p + numGroups;
+    RYO_CUDA(cudaMemsetAsync(gm2p, 0, 2 * sizeof(uint32_t) * size_t(numGroups), s));
     t.groupM2P      = gm2p;
     t.groupP2P      = gp2p;
     double pot = 0;
@@ -1542,10 +1554,8 @@ void solveSingle(ryo_ctx* ctx, const ryo_solve_params* P, float* x, float* y, fl
     {
         if (!(dbox.len[0] == dbox.len[1] && dbox.len[1] == dbox.len[2]))
             throw ApiError{RYO_ERR_NOT_CUBIC, "solve: Ewald needs a cubic periodic box"};
-        double hr[16];
-        RYO_CUDA(cudaMemcpyAsync(hr, root, sizeof(double) * 11, cudaMemcpyDeviceToHost, s));
-        RYO_CUDA(cudaStreamSynchronize(s));
-        EwaldHost e = ewaldSetup(hr + 3, hr, P->ewald.numReplicaShells, double(dbox.len[0]),
+        const double* hr = ctx->results->root; // the traversal has waited
+        EwaldHost e      = ewaldSetup(hr + 3, hr, P->ewald.numReplicaShells, double(dbox.len[0]),
                                  P->ewald.lCut, P->ewald.hCut, P->ewald.alpha_scale,
                                  P->ewald.small_R_scale_factor);
         double* ep = &ctx->ctl->ewaldPotential;
@@ -1608,10 +1618,8 @@ void solveSingle(ryo_ctx* ctx, const ryo_solve_params* P, float* x, float* y, fl
         a.groupP2P          = gp2p;
         a.dipoles           = reinterpret_cast<const float*>(dipoles);
         for (int i = 0; i < kMaxLevel + 2; ++i)
-            a.levelRange[i] = levelRange[i];
-        double hr[11];
-        RYO_CUDA(cudaMemcpyAsync(hr, root, sizeof(hr), cudaMemcpyDeviceToHost, s));
-        RYO_CUDA(cudaStreamSynchronize(s));
+            a.levelRange[i] = ctx->results->levelRange[i];
+        const double* hr = ctx->results->root;
         for (int i = 0; i < 3; ++i)
             a.rootCenter[i] = hr[i];
         for (int i = 0; i < 8; ++i)
@@ -1621,7 +1629,6 @@ void solveSingle(ryo_ctx* ctx, const ryo_solve_params* P, float* x, float* y, fl
     }
     if (ctx->hostStats[kMaxP2P] == 0xFFFFFFFFull)
         throw ApiError{RYO_ERR_STACK_OVERFLOW_UNSPLITTABLE, "solve: a single target overflowed"};
-    checkDeviceError(ctx, s);
     if (stats)
     {
         stats->numLeaves       = nl;
@@ -1757,22 +1764,25 @@ extern "C" ryo_status ryo_solve_batch_f32(ryo_ctx_t* ctx, const ryo_solve_params
                        mark(ctx, P, 0, s);
 
                        // per-system tables
-                       uint64_t* dFirst   = ctx->scratch<uint64_t>("batch.first", ns + 1, s);
-                       int* dUseGiven     = ctx->scratch<int>("batch.useGiven", ns, s);
-                       int* dShells       = ctx->scratch<int>("batch.shells", ns, s);
-                       DevBox<float>* dBx = ctx->scratch<DevBox<float>>("batch.boxes", ns, s);
-                       uint32_t* dGOff    = ctx->scratch<uint32_t>("batch.groupOffset", ns + 1, s);
+                       // one block and one copy: first bodies, group offsets, flags, shells and boxes
+                       const size_t atGOff = 8 * (size_t(ns) + 1), atGiven = atGOff + 4 * (size_t(ns) + 1),
+                                    atShells = atGiven + 4 * size_t(ns), atBoxes = atShells + 4 * size_t(ns);
+                       std::vector<char> tables(atBoxes + ns * sizeof(DevBox<float>));
+                       std::memcpy(tables.data(), first.data(), atGOff);
+                       std::memcpy(tables.data() + atGOff, groupOffset.data(), 4 * (size_t(ns) + 1));
+                       std::memcpy(tables.data() + atGiven, useGiven.data(), 4 * size_t(ns));
+                       std::memcpy(tables.data() + atShells, shells.data(), 4 * size_t(ns));
+                       std::memcpy(tables.data() + atBoxes, hbox.data(), ns * sizeof(DevBox<float>));
+                       static_assert(alignof(DevBox<float>) == 4, "the boxes start at a multiple of four bytes");
+                       char* dTables      = ctx->scratch<char>("batch.tables", tables.size(), s);
+                       uint64_t* dFirst   = reinterpret_cast<uint64_t*>(dTables);
+                       uint32_t* dGOff    = reinterpret_cast<uint32_t*>(dTables + atGOff);
+                       int* dUseGiven     = reinterpret_cast<int*>(dTables + atGiven);
+                       int* dShells       = reinterpret_cast<int*>(dTables + atShells);
+                       DevBox<float>* dBx = reinterpret_cast<DevBox<float>*>(dTables + atBoxes);
                        uint32_t* dMM      = ctx->scratch<uint32_t>("batch.minmax", 6 * size_t(ns), s);
                        float* dLimits     = ctx->scratch<float>("batch.limits", 6 * size_t(ns), s);
-                       RYO_CUDA(cudaMemcpyAsync(dFirst, first.data(), sizeof(uint64_t) * (ns + 1),
-                                                cudaMemcpyHostToDevice, s));
-                       RYO_CUDA(cudaMemcpyAsync(dUseGiven, useGiven.data(), sizeof(int) * ns, cudaMemcpyHostToDevice,
-                                                s));
-                       RYO_CUDA(cudaMemcpyAsync(dShells, shells.data(), sizeof(int) * ns, cudaMemcpyHostToDevice, s));
-                       RYO_CUDA(cudaMemcpyAsync(dBx, hbox.data(), sizeof(DevBox<float>) * ns, cudaMemcpyHostToDevice,
-                                                s));
-                       RYO_CUDA(cudaMemcpyAsync(dGOff, groupOffset.data(), sizeof(uint32_t) * (ns + 1),
-                                                cudaMemcpyHostToDevice, s));
+                       RYO_CUDA(cudaMemcpyAsync(dTables, tables.data(), tables.size(), cudaMemcpyHostToDevice, s));
                        launchBatchBoxes(x, y, z, n, dFirst, ns, dUseGiven, dMM, dBx, dLimits, s);
 
                        // system-prefixed keys, one sort for all systems, permute every per-body array
@@ -1874,9 +1884,8 @@ extern "C" ryo_status ryo_solve_batch_f32(ryo_ctx_t* ctx, const ryo_solve_params
                        launchBatchSofteningRange(h, dipoles ? nullptr : m, dFirst, ns, dTrav, s);
                        double* sysPot = ctx->scratch<double>("batch.pot", 2 * size_t(ns), s); // tree, Ewald
                        RYO_CUDA(cudaMemsetAsync(sysPot, 0, sizeof(double) * 2 * ns, s));
-                       for (float* a : {p, ax, ay, az})
-                           RYO_CUDA(cudaMemsetAsync(a, 0, n * sizeof(float), s));
                        TraverseLaunch t{};
+                       t.overwrite     = 1; // every body is in one group
                        t.groupStart    = tStart;
                        t.groupEnd      = tEnd;
                        t.numGroups     = int(travGroups);

@@ -471,7 +471,8 @@ template<class Kernel>
 unsigned residentBlocks(Kernel kernel, size_t smem, size_t warps, int smCount)
 {
     int perSm = 0;
-    RYO_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+    if (smem > 48 * 1024)
+        RYO_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
     RYO_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, kernel, kTravThreads, smem));
     return unsigned(std::min((warps + kTravWarps - 1) / kTravWarps, size_t(std::max(perSm, 1)) * smCount));
 }

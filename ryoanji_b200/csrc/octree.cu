@@ -22,6 +22,10 @@ namespace ryo
 {
 
 constexpr int kLeafBlock = 256;
+// keys up to which the leaves are sized by the keys instead of by a wait for the number of non-empty leaves: a solve of
+// 4,096 bodies 340 -> 333 us, of 2^18 bodies 1.817 -> 1.808 ms. At 2^20 the scan over a slot per key takes as long as the
+// wait (7.32 ms either way), and its buffers 25 bytes per key.
+constexpr uint32_t kOneWaitKeys = 1u << 18;
 
 /*! level of the leaf that contains each sorted particle, and where each particle starts a new non-empty leaf
  *
@@ -139,24 +143,31 @@ __global__ void __launch_bounds__(kLeafBlock) leafCompact(const uint64_t* __rest
     leafFirst[q]     = i;
 }
 
-//! number of output leaves contributed by non-empty leaf q: the gap before it plus itself (q == numNE: final gap)
-__global__ void leafSlots(const uint64_t* __restrict__ leafStart, const uint8_t* __restrict__ leafLvl, uint32_t numNE,
-                          uint32_t* __restrict__ slots)
+//! number of output leaves contributed by non-empty leaf q: the gap before it plus itself (q == numNE: final gap);
+//! none for the slots behind them, up to @p numSlots
+__global__ void leafSlots(const uint64_t* __restrict__ leafStart, const uint8_t* __restrict__ leafLvl,
+                          const uint32_t* __restrict__ numNonEmpty, uint32_t numSlots, uint32_t* __restrict__ slots)
 {
-    uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q > numNE) return;
+    const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x, numNE = *numNonEmpty;
+    if (q >= numSlots) return;
+    if (q > numNE)
+    {
+        slots[q] = 0;
+        return;
+    }
     uint64_t prevEnd = q == 0 ? 0 : leafStart[q - 1] + nodeRange(leafLvl[q - 1]);
     uint64_t start   = q == numNE ? kKeyEnd : leafStart[q];
     slots[q]         = uint32_t(spanKeyRange(prevEnd, start, nullptr)) + (q < numNE ? 1u : 0u);
 }
 
+//! the leaves, if @p capacity holds all offsets[numSlots] of them
 __global__ void leafWrite(const uint64_t* __restrict__ leafStart, const uint8_t* __restrict__ leafLvl,
-                          const uint32_t* __restrict__ leafFirst, const uint32_t* __restrict__ offsets, uint32_t numNE,
-                          uint32_t n, uint64_t* __restrict__ leaves, uint32_t* __restrict__ counts,
-                          uint32_t* __restrict__ layout)
+                          const uint32_t* __restrict__ leafFirst, const uint32_t* __restrict__ offsets,
+                          const uint32_t* __restrict__ numNonEmpty, uint32_t numSlots, int64_t capacity, uint32_t n,
+                          uint64_t* __restrict__ leaves, uint32_t* __restrict__ counts, uint32_t* __restrict__ layout)
 {
-    uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q > numNE) return;
+    const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x, numNE = *numNonEmpty;
+    if (q > numNE || int64_t(offsets[numSlots]) > capacity) return;
     uint64_t prevEnd = q == 0 ? 0 : leafStart[q - 1] + nodeRange(leafLvl[q - 1]);
     uint64_t start   = q == numNE ? kKeyEnd : leafStart[q];
     uint32_t o       = offsets[q];
@@ -220,29 +231,34 @@ int buildLeaves(ryo_ctx* ctx, const uint64_t* keys, size_t n64, unsigned bucket,
     leafLevels<<<numBlocks, kLeafBlock, smemBytes, s>>>(keys, n, bucket, minLevel, level, head, blockHeads);
     RYO_LAUNCH_CHECK();
     exclusiveScanU32(ctx, blockHeads, blockHeads, numBlocks, s);
-    uint32_t numNE = 0;
-    RYO_CUDA(cudaMemcpyAsync(&numNE, blockHeads + numBlocks, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-    RYO_CUDA(cudaStreamSynchronize(s));
-
-    uint64_t* leafStart = ctx->scratch<uint64_t>("leaf.start", numNE, s);
-    uint8_t* leafLvl    = ctx->scratch<uint8_t>("leaf.lvl", numNE, s);
-    uint32_t* leafFirst = ctx->scratch<uint32_t>("leaf.first", numNE, s);
-    uint32_t* slots     = ctx->scratch<uint32_t>("leaf.slots", size_t(numNE) + 2, s);
+    const uint32_t* numNonEmpty = blockHeads + numBlocks;
+    // the host sizes what follows by the number of non-empty leaves, for few keys by the number of keys
+    uint32_t most = n;
+    if (n > kOneWaitKeys)
+    {
+        RYO_CUDA(cudaMemcpyAsync(&ctx->results->count, numNonEmpty, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+        RYO_CUDA(cudaStreamSynchronize(s));
+        most = ctx->results->count;
+    }
+    const uint32_t numSlots = most + 1;
+    uint64_t* leafStart     = ctx->scratch<uint64_t>("leaf.start", most, s);
+    uint8_t* leafLvl        = ctx->scratch<uint8_t>("leaf.lvl", most, s);
+    uint32_t* leafFirst     = ctx->scratch<uint32_t>("leaf.first", most, s);
+    uint32_t* slots         = ctx->scratch<uint32_t>("leaf.slots", size_t(numSlots) + 1, s);
     leafCompact<<<numBlocks, kLeafBlock, 0, s>>>(keys, level, head, blockHeads, n, leafStart, leafLvl, leafFirst);
     RYO_LAUNCH_CHECK();
-    leafSlots<<<ceilDiv(numNE + 1, 256), 256, 0, s>>>(leafStart, leafLvl, numNE, slots);
+    leafSlots<<<ceilDiv(numSlots, 256), 256, 0, s>>>(leafStart, leafLvl, numNonEmpty, numSlots, slots);
     RYO_LAUNCH_CHECK();
-    exclusiveScanU32(ctx, slots, slots, size_t(numNE) + 1, s);
-    uint32_t numLeaves = 0;
-    RYO_CUDA(cudaMemcpyAsync(&numLeaves, slots + numNE + 1, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-    RYO_CUDA(cudaStreamSynchronize(s));
-    if (int64_t(numLeaves) <= int64_t(capacity))
+    exclusiveScanU32(ctx, slots, slots, numSlots, s);
+    RYO_CUDA(cudaMemcpyAsync(&ctx->results->count, slots + numSlots, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+    if (leaves && counts)
     {
-        leafWrite<<<ceilDiv(numNE + 1, 256), 256, 0, s>>>(leafStart, leafLvl, leafFirst, slots, numNE, n, leaves,
-                                                           counts, layout);
+        leafWrite<<<ceilDiv(numSlots, 256), 256, 0, s>>>(leafStart, leafLvl, leafFirst, slots, numNonEmpty, numSlots,
+                                                          capacity, n, leaves, counts, layout);
         RYO_LAUNCH_CHECK();
     }
-    return int(numLeaves);
+    RYO_CUDA(cudaStreamSynchronize(s));
+    return int(ctx->results->count);
 }
 
 // ------------------------------------------------------------------------------------------------ links
@@ -396,8 +412,11 @@ void linkOctree(ryo_ctx* ctx, const uint64_t* leaves, int numLeaves, const Octre
                                                              out.childOffsets, out.parents);
         RYO_LAUNCH_CHECK();
     }
-    RYO_CUDA(cudaMemcpyAsync(hostLevelRange, dlr, sizeof(int) * (kMaxLevel + 2), cudaMemcpyDeviceToHost, s));
+    int* range = ctx->results->levelRange;
+    RYO_CUDA(cudaMemcpyAsync(range, dlr, sizeof(int) * (kMaxLevel + 2), cudaMemcpyDeviceToHost, s));
+    if (!hostLevelRange) return;
     RYO_CUDA(cudaStreamSynchronize(s));
+    std::copy(range, range + kMaxLevel + 2, hostLevelRange);
 }
 
 // ------------------------------------------------------------------------------------------------ groups

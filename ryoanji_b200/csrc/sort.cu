@@ -110,8 +110,45 @@ __global__ void __launch_bounds__(kScanBlock) scanApply(const uint32_t* in, size
     if (blockIdx.x == 0 && threadIdx.x == 0) out[n] = tileOffsets[numTiles];
 }
 
+//! the whole scan of a few tiles in one block
+__global__ void __launch_bounds__(kScanBlock) scanOneBlock(const uint32_t* in, uint32_t n, uint32_t* out)
+{
+    __shared__ uint32_t sWarp[32];
+    uint32_t carry = 0;
+    for (uint32_t tile = 0; tile < n; tile += kScanTile)
+    {
+        const uint32_t base = tile + threadIdx.x * kScanItems;
+        uint32_t v[kScanItems], sum = 0, total;
+#pragma unroll
+        for (int i = 0; i < kScanItems; ++i)
+        {
+            v[i] = base + i < n ? in[base + i] : 0;
+            sum += v[i];
+        }
+        uint32_t run = carry + blockInclusiveScan(sum, sWarp, &total) - sum;
+#pragma unroll
+        for (int i = 0; i < kScanItems; ++i)
+        {
+            if (base + i < n) out[base + i] = run;
+            run += v[i];
+        }
+        carry += total;
+    }
+    if (threadIdx.x == 0) out[n] = carry;
+}
+
+// values that one block scans in one launch instead of three: the two scans of a solve of 4,096 bodies 18 us less, of
+// 60,001 bodies 15 us less. With 16 tiles the latter's took 25 us more than with three launches.
+constexpr size_t kScanOneBlock = 4 * size_t(kScanTile);
+
 void exclusiveScanU32(ryo_ctx* ctx, const uint32_t* in, uint32_t* out, size_t n, cudaStream_t s)
 {
+    if (n > 0 && n <= kScanOneBlock)
+    {
+        scanOneBlock<<<1, kScanBlock, 0, s>>>(in, uint32_t(n), out);
+        RYO_LAUNCH_CHECK();
+        return;
+    }
     uint32_t numTiles = uint32_t((n + kScanTile - 1) / kScanTile);
     if (numTiles == 0)
     {
