@@ -1881,7 +1881,7 @@ extern "C" ryo_status ryo_solve_batch_f32(ryo_ctx_t* ctx, const ryo_solve_params
                                         oct.childOffsets, sysLevel, dBx, dShells, dTrav, dRootNode, rootErr, s);
                        // the mass range only where quadrupoles are summed (signed-mass expansions keep the
                        // per-source mass)
-                       launchBatchSofteningRange(h, dipoles ? nullptr : m, dFirst, ns, dTrav, s);
+                       launchBatchSofteningRange(h, dipoles ? nullptr : m, n, dFirst, ns, dTrav, s);
                        double* sysPot = ctx->scratch<double>("batch.pot", 2 * size_t(ns), s); // tree, Ewald
                        RYO_CUDA(cudaMemsetAsync(sysPot, 0, sizeof(double) * 2 * ns, s));
                        TraverseLaunch t{};

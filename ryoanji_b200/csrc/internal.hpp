@@ -437,9 +437,9 @@ struct SysTrav
     uint32_t hLo, hHi; // min and max softening of the system's bodies as ordered bits (hLo > hHi: not known)
     uint32_t mLo, mHi; // min and max mass of the system's bodies as ordered bits (mLo > mHi: not known)
 };
-//! per-system softening and mass ranges of a batched solve into trav[s].hLo / hHi / mLo / mHi (one block per
-//! system); m may be null (the mass range then stays unknown)
-void launchBatchSofteningRange(const float* h, const float* m, const uint64_t* first, uint32_t numSystems,
+//! per-system softening and mass ranges of a batched solve into trav[s].hLo / hHi / mLo / mHi, which hold
+//! the neutral values; m may be null (the mass range then stays unknown)
+void launchBatchSofteningRange(const float* h, const float* m, size_t n, const uint64_t* first, uint32_t numSystems,
                                SysTrav* trav, cudaStream_t s);
 void launchTraverse(const TraverseLaunch& t, int smCount, cudaStream_t s);
 //! what a reset clears: the statistics and all counters, a pass's counters, or those of the interaction lists

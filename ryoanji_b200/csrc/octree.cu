@@ -22,9 +22,9 @@ namespace ryo
 {
 
 constexpr int kLeafBlock = 256;
-// keys up to which the leaves are sized by the keys instead of by a wait for the number of non-empty leaves: a solve of
-// 4,096 bodies 340 -> 333 us, of 2^18 bodies 1.817 -> 1.808 ms. At 2^20 the scan over a slot per key takes as long as the
-// wait (7.32 ms either way), and its buffers 25 bytes per key.
+// keys up to which the leaves are sized by the keys instead of by a wait for the number of non-empty leaves: a solve
+// of 4,096 bodies 340 -> 333 us, of 2^18 bodies 1.817 -> 1.808 ms. At 2^20 the scan over a slot per key takes as long
+// as the wait (7.32 ms either way), and its buffers 25 bytes per key.
 constexpr uint32_t kOneWaitKeys = 1u << 18;
 
 /*! level of the leaf that contains each sorted particle, and where each particle starts a new non-empty leaf
