@@ -572,7 +572,11 @@ __global__ void splitGroupsKernel(const uint32_t* failed, uint32_t numFailed, co
 constexpr uint32_t kListGroups  = 49152;
 constexpr uint32_t kSubGroups   = 6000;  // groups up to which every list walk is split into eight parts
 constexpr size_t kListBytes     = size_t(512) << 20; // of list items
-constexpr unsigned kMinItemCost = 1024;  // 16 evaluation batches
+// interactions of an item: half the groups' number, at least 1024 (16 evaluation batches), below 512 groups twice their
+// number, so that the items of the smallest solves still number as many as the GPU has warps: 1,000 bodies 303 -> 267
+// us, the traversal of 4,096 bodies 105 -> 95 us, of 16,384 bodies 203 -> 193 us. Four times their number is slower
+// between 128 and 512 groups (16,384 bodies 202 us).
+constexpr unsigned kMinItemCost = 1024;
 constexpr unsigned kMaxItemCost = 16384;
 constexpr unsigned kHeavyCost   = 32768; // of the fused kernel's groups; compact ones cost about 17,000 at most
 
@@ -611,7 +615,7 @@ void traverseLists(ryo_ctx* ctx, TraverseLaunch t, const uint32_t* list, uint32_
     const uint32_t numGroups = uint32_t(t.numGroups);
     // a caller's stack capacity is for one walk of the whole tree
     t.subWalks  = (list || solveGroups <= kSubGroups) && ownStack ? 8 : 1;
-    t.itemCost  = std::min(kMaxItemCost, std::max(kMinItemCost, solveGroups / 2));
+    t.itemCost  = std::min(kMaxItemCost, std::max(std::min(kMinItemCost, 2 * solveGroups), solveGroups / 2));
     t.itemWords = t.subWalks > 1 ? 512 : 2048;
     const size_t tasks = size_t(count) * t.subWalks;
     // pieces per part of a walk seldom pass this; when they do, the groups that found no room walk again
