@@ -575,7 +575,8 @@ constexpr size_t kListBytes     = size_t(512) << 20; // of list items
 // interactions of an item: half the groups' number, at least 1024 (16 evaluation batches), below 512 groups twice their
 // number, so that the items of the smallest solves still number as many as the GPU has warps: 1,000 bodies 303 -> 267
 // us, the traversal of 4,096 bodies 105 -> 95 us, of 16,384 bodies 203 -> 193 us. Four times their number is slower
-// between 128 and 512 groups (16,384 bodies 202 us).
+// between 128 and 512 groups (16,384 bodies 202 us). A batched solve keeps 1024, so that a small system's sums are the
+// same alone and among others.
 constexpr unsigned kMinItemCost = 1024;
 constexpr unsigned kMaxItemCost = 16384;
 constexpr unsigned kHeavyCost   = 32768; // of the fused kernel's groups; compact ones cost about 17,000 at most
@@ -615,7 +616,8 @@ void traverseLists(ryo_ctx* ctx, TraverseLaunch t, const uint32_t* list, uint32_
     const uint32_t numGroups = uint32_t(t.numGroups);
     // a caller's stack capacity is for one walk of the whole tree
     t.subWalks  = (list || solveGroups <= kSubGroups) && ownStack ? 8 : 1;
-    t.itemCost  = std::min(kMaxItemCost, std::max(std::min(kMinItemCost, 2 * solveGroups), solveGroups / 2));
+    const unsigned minCost = t.groupSys ? kMinItemCost : std::min(kMinItemCost, 2 * solveGroups);
+    t.itemCost  = std::min(kMaxItemCost, std::max(minCost, solveGroups / 2));
     t.itemWords = t.subWalks > 1 ? 512 : 2048;
     const size_t tasks = size_t(count) * t.subWalks;
     // pieces per part of a walk seldom pass this; when they do, the groups that found no room walk again
