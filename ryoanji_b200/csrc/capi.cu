@@ -616,6 +616,7 @@ void traverseLists(ryo_ctx* ctx, TraverseLaunch t, const uint32_t* list, uint32_
     const uint32_t numGroups = uint32_t(t.numGroups);
     // a caller's stack capacity is for one walk of the whole tree
     t.subWalks  = (list || solveGroups <= kSubGroups) && ownStack ? 8 : 1;
+    t.walkEntries = ownStack ? 8 : 4; // two steps at once need more stack, which a caller may have sized for one
     const unsigned minCost = t.groupSys ? kMinItemCost : std::min(kMinItemCost, 2 * solveGroups);
     t.itemCost  = std::min(kMaxItemCost, std::max(minCost, solveGroups / 2));
     t.itemWords = t.subWalks > 1 ? 512 : 2048;

@@ -390,6 +390,7 @@ struct TraverseLaunch
     // else the interaction-list kernels, for all groups or those in groupList: walks in subWalks parts (1, or 8) write
     // items of itemWords words, closed past itemCost interactions
     uint32_t subWalks;
+    int walkEntries;        // stack entries that a float list walk takes at once: 4, or 8 for two steps
     const uint32_t* groupList;
     ListItem* items;
     uint32_t* lists;

@@ -5,8 +5,10 @@
  * group's items in a fixed order. The time of a small solve is then that of its total work and not of its longest
  * group's. The walk follows the reference's rule (ryoanji/src/ryoanji/nbody/traversal_gpu.cu:210-237).
  *
- * What bounds it: the walk is bound by instruction issue (a step of 32 cells takes about 100 instructions, 4-6% of the
- * evaluation's time); its lists take 6-15 KB per group and stay in the L2 between the two kernels.
+ * What bounds it: the walk of many groups is bound by instruction issue and the L1 (a step of 32 cells takes about 170
+ * instructions with the list's writing; 5% of the evaluation's time), that of few groups by the latency of its longest
+ * part. Two steps' cells loaded at once: 2^20 Plummer bodies 398 -> 338 us, 60,001 bodies 132 -> 112 us. The lists take
+ * 6-15 KB per group and stay in the L2 between the two kernels.
  */
 #pragma once
 
@@ -195,6 +197,9 @@ __device__ __forceinline__ bool walkTask(const TraverseLaunch& P, const Nodes& n
     const int b = int(P.groupStart[g]), e = int(P.groupEnd[g]);
     using R = typename Nodes::Real;
     using F = Fp<R>;
+    // steps whose cells are loaded at once; in double a second one costs more registers than the latency is worth (the
+    // walk of 120,001 Plummer bodies 88 -> 100 us)
+    constexpr int kSteps = std::is_same_v<R, float> ? 2 : 1;
     R tc[3], ts[3];
     {
         R u[3], v[3];
@@ -246,77 +251,94 @@ __device__ __forceinline__ bool walkTask(const TraverseLaunch& P, const Nodes& n
                 __syncwarp();
                 if (lane == 0) stack[0] = start;
                 __syncwarp();
-                while (sp > 0 && !L.starved)
+                while (sp > 0 && !L.starved && !overflow)
                 {
-                    int k     = min(4, sp);
+                    // four stack entries, 32 cells, per step; the next step's cells are loaded with them, so that two
+                    // steps wait for the L2 once
+                    const int k = min(kSteps > 1 ? P.walkEntries : 4, sp);
                     sp -= k;
-                    int slot  = lane >> 3;
-                    int entry = slot < k ? stack[sp + slot] : -1;
+                    const int slot = lane >> 3;
+                    int cells[kSteps];
+                    typename Nodes::Center centers[kSteps] = {};
+                    int4 links[kSteps]                     = {};
+#pragma unroll
+                    for (int u = 0; u < kSteps; ++u)
+                    {
+                        const int at    = k - 4 * (u + 1) + slot; // from the top down
+                        const int entry = at >= 0 && at < k - 4 * u ? stack[sp + at] : -1;
+                        cells[u]        = -1;
+                        if (entry <= kRootOnly) cells[u] = (lane & 7) == 0 ? kRootOnly - entry : -1;
+                        else if (entry >= 0) cells[u] = entry + (lane & 7);
+                    }
                     __syncwarp();
-                    int cell = -1;
-                    if (entry <= kRootOnly) cell = (lane & 7) == 0 ? kRootOnly - entry : -1;
-                    else if (entry >= 0) cell = entry + (lane & 7);
-
-                    bool valid = cell >= 0;
-                    typename Nodes::Center c{};
-                    int4 link = make_int4(0, 0, 0, 0);
-                    if (valid) nodes.load(cell, c, link);
-                    bool close  = valid && macFails(c, tc, ts);
-                    bool isNode = link.x != 0;
-                    bool split  = close && isNode;
-                    unsigned bs = __ballot_sync(0xffffffffu, split);
-                    int nsplit  = __popc(bs);
-                    if (sp + nsplit > P.stackCapacity)
+#pragma unroll
+                    for (int u = 0; u < kSteps; ++u)
+                        if (cells[u] >= 0) nodes.load(cells[u], centers[u], links[u]);
+#pragma unroll
+                    for (int u = 0; u < kSteps; ++u)
                     {
-                        overflow = true;
-                        break;
-                    }
-                    if (split) stack[sp + __popc(bs & lt)] = link.x;
-                    sp += nsplit;
-                    maxStack = max(maxStack, sp);
-
-                    bool direct = close && !isNode;
-                    bool remote = direct && link.z == 0 && c.w != R(0);
-                    bool approx = valid && (!close || remote);
-                    nM2P += approx ? 1u : 0u;
-
-                    bool evalM  = approx && c.w != R(0); // massless cells contribute exactly zero
-                    unsigned bm = __ballot_sync(0xffffffffu, evalM);
-                    if (evalM)
-                    {
-                        W.m2p[nM + __popc(bm & lt)] = cell;
-                        if (images) W.image[nM + __popc(bm & lt)] = image;
-                    }
-                    nM += __popc(bm);
-
-                    bool hasB   = direct && link.z > 0;
-                    unsigned bl = __ballot_sync(0xffffffffu, hasB);
-                    if (hasB)
-                    {
-                        W.leaves[nL + __popc(bl & lt)] = make_int2(link.y, link.z);
-                        nP2P += unsigned(link.z);
-                    }
-                    nL += __popc(bl);
-                    __syncwarp();
-                    if (nM >= kM2PCap)
-                    {
-                        L.cells(P, g, W, kM2PCap, images, replicas && !images ? rep : nullptr);
-                        nM -= kM2PCap; // fewer than kWarp cells remain: one move per lane
-                        __syncwarp();
-                        if (lane < nM)
+                        if (4 * u >= k) break;
+                        const int cell                 = cells[u];
+                        const bool valid               = cell >= 0;
+                        const typename Nodes::Center c = centers[u];
+                        const int4 link                = links[u];
+                        bool close  = valid && macFails(c, tc, ts);
+                        bool isNode = link.x != 0;
+                        bool split  = close && isNode;
+                        unsigned bs = __ballot_sync(0xffffffffu, split);
+                        int nsplit  = __popc(bs);
+                        if (sp + nsplit > P.stackCapacity)
                         {
-                            W.m2p[lane] = W.m2p[kM2PCap + lane];
-                            if (images) W.image[lane] = W.image[kM2PCap + lane];
+                            overflow = true;
+                            break;
                         }
+                        if (split) stack[sp + __popc(bs & lt)] = link.x;
+                        sp += nsplit;
+                        maxStack = max(maxStack, sp);
+
+                        bool direct = close && !isNode;
+                        bool remote = direct && link.z == 0 && c.w != R(0);
+                        bool approx = valid && (!close || remote);
+                        nM2P += approx ? 1u : 0u;
+
+                        bool evalM  = approx && c.w != R(0); // massless cells contribute exactly zero
+                        unsigned bm = __ballot_sync(0xffffffffu, evalM);
+                        if (evalM)
+                        {
+                            W.m2p[nM + __popc(bm & lt)] = cell;
+                            if (images) W.image[nM + __popc(bm & lt)] = image;
+                        }
+                        nM += __popc(bm);
+
+                        bool hasB   = direct && link.z > 0;
+                        unsigned bl = __ballot_sync(0xffffffffu, hasB);
+                        if (hasB)
+                        {
+                            W.leaves[nL + __popc(bl & lt)] = make_int2(link.y, link.z);
+                            nP2P += unsigned(link.z);
+                        }
+                        nL += __popc(bl);
                         __syncwarp();
-                    }
-                    if (nL >= kSegLeafCap)
-                    {
-                        L.leaves(P, g, W, kSegLeafCap, replicas ? rep : nullptr);
-                        nL -= kSegLeafCap;
-                        __syncwarp();
-                        if (lane < nL) W.leaves[lane] = W.leaves[kSegLeafCap + lane];
-                        __syncwarp();
+                        if (nM >= kM2PCap)
+                        {
+                            L.cells(P, g, W, kM2PCap, images, replicas && !images ? rep : nullptr);
+                            nM -= kM2PCap; // fewer than kWarp cells remain: one move per lane
+                            __syncwarp();
+                            if (lane < nM)
+                            {
+                                W.m2p[lane] = W.m2p[kM2PCap + lane];
+                                if (images) W.image[lane] = W.image[kM2PCap + lane];
+                            }
+                            __syncwarp();
+                        }
+                        if (nL >= kSegLeafCap)
+                        {
+                            L.leaves(P, g, W, kSegLeafCap, replicas ? rep : nullptr);
+                            nL -= kSegLeafCap;
+                            __syncwarp();
+                            if (lane < nL) W.leaves[lane] = W.leaves[kSegLeafCap + lane];
+                            __syncwarp();
+                        }
                     }
                 }
                 overflow |= L.starved;
