@@ -497,6 +497,16 @@ __device__ void combineChildren(const FusedArgs& A, int node, int fc, int sub, u
     }
 }
 
+//! counts an arrival at @p counter: the caller's writes are seen by who arrives later, and it sees theirs who came
+//! before. A climb is a chain of such arrivals; with full fences on both sides of the count an upsweep took 31.5
+//! instead of 28 us for 4,096 bodies and 82 instead of 77 us for 2^20.
+__device__ __forceinline__ unsigned arrive(unsigned int* counter)
+{
+    unsigned old;
+    asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(old) : "l"(counter) : "memory");
+    return old;
+}
+
 /*! eight lanes per leaf: one pass over the bodies, P2M of the leaf (small register footprint, so many leaf groups
  *  stay resident per SM). The internal nodes follow by the climb (A.arrivals set: the group of the eighth sibling to
  *  arrive combines the parent, one child per lane, and goes on up) or level by level (levelCombineKernel). */
@@ -601,12 +611,11 @@ __global__ void __launch_bounds__(256, 4) fusedUpsweepKernel(FusedArgs A)
         int last   = 0;
         if (sub == 0)
         {
-            __threadfence();
-            last = atomicAdd(A.arrivals + parent, 1u) == 7u;
+            last = arrive(A.arrivals + parent) == 7u;
         }
         last = __shfl_sync(gmask, last, 0, kTpl);
         if (!last) break;
-        __threadfence();
+        __syncwarp(gmask); // what lane 0 has seen written, all lanes have
         combineChildren(A, parent, A.childOffsets[parent], sub, gmask);
         node = parent;
     }
