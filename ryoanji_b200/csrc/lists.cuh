@@ -414,32 +414,42 @@ __global__ void __launch_bounds__(kTravThreads) walkKernel(TraverseLaunch P, Nod
 }
 
 constexpr int kFinishThreads = 256;
+constexpr int kWalkParts     = kFinishThreads / kWarp; // parts of a divided walk
 
-/*! every group of the launch, one warp each: interaction counts and statistics, and the results of the groups whose
- *  list became items (or is empty): the items' sums added in FP64 in a fixed order. @p sink reads the items' sums and
- *  stores a target's results, returning its m phi. */
-template<class Sink>
+/*! every group of the launch: interaction counts and statistics, and the results of the groups whose list became items
+ *  (or is empty): the items' sums added in FP64 in a fixed order. @p sink reads the items' sums and stores a target's
+ *  results, returning its m phi. Bound by the latency of the chains of items: a warp follows those of a group's parts one
+ *  after the other, with kParts the warps of a block at once. */
+template<bool kParts, class Sink>
 __global__ void __launch_bounds__(kFinishThreads) finishKernel(TraverseLaunch P, Sink sink)
 {
-    const int lane        = laneId();
-    const unsigned stride = gridDim.x * (kFinishThreads / kWarp);
+    const int lane = laneId(), warp = threadIdx.x / kWarp;
+    const unsigned stride = kParts ? gridDim.x : gridDim.x * (kFinishThreads / kWarp);
+    __shared__ double sPart[kParts ? kWalkParts : 1][4][2 * kWarp];
     unsigned long long sumP = 0, sumM = 0, maxP = 0, maxM = 0;
-    for (unsigned i = (blockIdx.x * kFinishThreads + threadIdx.x) / kWarp; i < unsigned(P.numGroups); i += stride)
+    for (unsigned i = kParts ? blockIdx.x : (blockIdx.x * kFinishThreads + threadIdx.x) / kWarp;
+         i < unsigned(P.numGroups); i += stride)
     {
         const unsigned g = P.groupList ? P.groupList[i] : i;
         if (P.groupState[g] != 0u) continue;
         const int b = int(P.groupStart[g]), e = int(P.groupEnd[g]);
-        const unsigned nM = P.countM2P[g], nP = P.countP2P[g];
-        sumP += (unsigned long long)nP * unsigned(e - b);
-        sumM += (unsigned long long)nM * unsigned(e - b);
-        maxP = max(maxP, (unsigned long long)nP);
-        maxM = max(maxM, (unsigned long long)nM);
-        if (lane == 0 && P.groupM2P) P.groupM2P[g] = nM;
-        if (lane == 0 && P.groupP2P) P.groupP2P[g] = nP;
+        if (!kParts || warp == 0)
+        {
+            const unsigned nM = P.countM2P[g], nP = P.countP2P[g];
+            sumP += (unsigned long long)nP * unsigned(e - b);
+            sumM += (unsigned long long)nM * unsigned(e - b);
+            maxP = max(maxP, (unsigned long long)nP);
+            maxM = max(maxM, (unsigned long long)nM);
+            if (lane == 0 && P.groupM2P) P.groupM2P[g] = nM;
+            if (lane == 0 && P.groupP2P) P.groupP2P[g] = nP;
+        }
         double sum[2][4] = {};
-        const int last   = P.taskLast[i * P.subWalks];
-        if (last >= 0 && P.items[last].only) continue;
-        for (unsigned sub = 0; sub < P.subWalks; ++sub)
+        if (!kParts)
+        {
+            const int last = P.taskLast[i * P.subWalks];
+            if (last >= 0 && P.items[last].only) continue;
+        }
+        for (unsigned sub = kParts ? warp : 0; sub < P.subWalks; sub += kParts ? kWalkParts : 1)
         {
             for (int it = P.taskLast[i * P.subWalks + sub]; it >= 0; it = P.items[it].prev)
             {
@@ -454,15 +464,37 @@ __global__ void __launch_bounds__(kFinishThreads) finishKernel(TraverseLaunch P,
                 }
             }
         }
+        if constexpr (kParts)
+        {
+#pragma unroll
+            for (int t = 0; t < 2; ++t)
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+                    sPart[warp][k][t * kWarp + lane] = sum[t][k];
+            __syncthreads();
+            if (warp < 2) // 32 targets each
+            {
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+                {
+                    sum[0][k] = 0.0;
+#pragma unroll
+                    for (int w = 0; w < kWalkParts; ++w)
+                        sum[0][k] += sPart[w][k][warp * kWarp + lane];
+                }
+            }
+            __syncthreads();
+            if (warp >= 2) continue;
+        }
         double pot = 0.0;
 #pragma unroll
-        for (int t = 0; t < 2; ++t)
+        for (int t = 0; t < (kParts ? 1 : 2); ++t)
         {
-            int idx = b + t * kWarp + lane;
+            const int idx = b + (kParts ? warp : t) * kWarp + lane;
             if (idx < e) pot += sink.store(P, idx, sum[t]);
         }
         pot = warpSum(pot);
-        if (lane == 0)
+        if (lane == 0 && pot != 0.0)
         {
             atomicAdd(&P.ctl->potential, pot);
             if (P.sysPotential) atomicAdd(P.sysPotential + (P.groupSys ? P.groupSys[g] : 0u), pot);
@@ -470,7 +502,6 @@ __global__ void __launch_bounds__(kFinishThreads) finishKernel(TraverseLaunch P,
     }
     // every lane of a warp holds the same counts; one set of atomics per block
     __shared__ unsigned long long sh[4][kFinishThreads / kWarp];
-    const int warp = threadIdx.x / kWarp;
     if (lane == 0) sh[0][warp] = sumP, sh[1][warp] = sumM, sh[2][warp] = maxP, sh[3][warp] = maxM;
     __syncthreads();
     if (threadIdx.x != 0) return;
@@ -512,8 +543,17 @@ void launchWalk(const TraverseLaunch& t, const Nodes& nodes, const Targets& tgt,
 template<class Sink>
 void launchFinish(const TraverseLaunch& t, const Sink& sink, int smCount, cudaStream_t s)
 {
-    const size_t blocks = ceilDiv(size_t(t.numGroups) * kWarp, kFinishThreads);
-    finishKernel<<<unsigned(std::min(blocks, size_t(8) * smCount)), kFinishThreads, 0, s>>>(t, sink);
+    // a block per group for as many groups as two rounds of eight blocks per SM take: the chains are long there (100,003
+    // bodies at theta 0.2, 1,563 groups: 81 -> 22 us; 60,001 Plummer bodies: 32 -> 17 us), but with 3,907 groups of a
+    // cube, whose parts are an item or two, it took 34 instead of 20 us
+    const size_t numGroups = size_t(t.numGroups);
+    if (t.subWalks == kWalkParts && numGroups <= size_t(16) * smCount)
+        finishKernel<true><<<unsigned(std::min(numGroups, size_t(8) * smCount)), kFinishThreads, 0, s>>>(t, sink);
+    else
+    {
+        const size_t blocks = ceilDiv(numGroups * kWarp, kFinishThreads);
+        finishKernel<false><<<unsigned(std::min(blocks, size_t(8) * smCount)), kFinishThreads, 0, s>>>(t, sink);
+    }
     RYO_LAUNCH_CHECK();
 }
 
