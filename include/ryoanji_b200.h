@@ -309,8 +309,7 @@ extern "C"
      * float, Tf = double, multipoles of floats), the caller side of codes whose particle positions are double. As in
      * the reference, the MAC and the sums run in double with the single-precision rsqrt of the double argument
      * (kernel.hpp:38-52). Centres are 4 doubles per node; multipoles 8 values per node, or 12 with options->multipole
-     * = RYO_MULTIPOLE_MDQ. Semantics, checks and statistics are those of ryo_traverse_ex_f32 (options may be NULL).
-     * A group too costly for one warp is evaluated by one warp here (no split second pass). */
+     * = RYO_MULTIPOLE_MDQ. Semantics, checks and statistics are those of ryo_traverse_ex_f32 (options may be NULL). */
     RYO_API ryo_status ryo_traverse_f64(ryo_ctx_t* ctx, const ryo_group_view* grp, int initNodeIdx, const double* xt,
                                         const double* yt, const double* zt, const double* mt, const double* ht,
                                         const double* xs, const double* ys, const double* zs, const double* ms,

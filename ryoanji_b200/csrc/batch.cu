@@ -32,12 +32,12 @@ __device__ __forceinline__ uint32_t systemOf(const uint64_t* __restrict__ first,
 
 constexpr int kRangeStep = 8 * kWarp; // bodies per round of a warp
 
-/*! per-system minima and maxima of kArrays arrays, as ordered bits: (min, max) of each array from @p out + s * @p stride
- *  on, which hold the neutral values at the start. A warp has @p chunk consecutive bodies and adds its result of every
- *  system among them with one atomic per value. With kSkipNaN NaNs are passed over, as by fminf and fmaxf. Bound by the
- *  latency of its loads and atomics. 2.7M bodies in 256 systems: coordinates 15 us, softenings and masses 10 us. With 64
- *  bodies in a row per thread, whose loads are not coalesced, the coordinates took 62 us; with a block per system, which
- *  waits for the largest, the softenings and masses 69 us. */
+/*! per-system minima and maxima of kArrays arrays, as ordered bits: (min, max) of each array from @p out + s *
+ *  @p stride on, which hold the neutral values at the start. A warp has @p chunk consecutive bodies and adds its result
+ *  of every system among them with one atomic per value. With kSkipNaN NaNs are passed over, as by fminf and fmaxf.
+ *  Bound by the latency of its loads and atomics. 2.7M bodies in 256 systems: coordinates 15 us, softenings and masses
+ *  10 us. With 64 bodies in a row per thread, whose loads are not coalesced, the coordinates took 62 us; with a block
+ *  per system, which waits for the largest, the softenings and masses 69 us. */
 template<int kArrays, bool kSkipNaN>
 __global__ void batchRangesKernel(const float* __restrict__ a0, const float* __restrict__ a1,
                                   const float* __restrict__ a2, size_t n, size_t chunk,

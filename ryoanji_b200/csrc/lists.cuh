@@ -418,8 +418,8 @@ constexpr int kWalkParts     = kFinishThreads / kWarp; // parts of a divided wal
 
 /*! every group of the launch: interaction counts and statistics, and the results of the groups whose list became items
  *  (or is empty): the items' sums added in FP64 in a fixed order. @p sink reads the items' sums and stores a target's
- *  results, returning its m phi. Bound by the latency of the chains of items: a warp follows those of a group's parts one
- *  after the other, with kParts the warps of a block at once. */
+ *  results, returning its m phi. Bound by the latency of the chains of items: a warp follows those of a group's parts
+ *  one after the other, with kParts the warps of a block at once. */
 template<bool kParts, class Sink>
 __global__ void __launch_bounds__(kFinishThreads) finishKernel(TraverseLaunch P, Sink sink)
 {
@@ -543,9 +543,9 @@ void launchWalk(const TraverseLaunch& t, const Nodes& nodes, const Targets& tgt,
 template<class Sink>
 void launchFinish(const TraverseLaunch& t, const Sink& sink, int smCount, cudaStream_t s)
 {
-    // a block per group for as many groups as two rounds of eight blocks per SM take: the chains are long there (100,003
-    // bodies at theta 0.2, 1,563 groups: 81 -> 22 us; 60,001 Plummer bodies: 32 -> 17 us), but with 3,907 groups of a
-    // cube, whose parts are an item or two, it took 34 instead of 20 us
+    // a block per group for as many groups as two rounds of eight blocks per SM take: the chains are long there
+    // (100,003 bodies at theta 0.2, 1,563 groups: 81 -> 22 us; 60,001 Plummer bodies: 32 -> 17 us), but with 3,907
+    // groups of a cube, whose parts are an item or two, it took 34 instead of 20 us
     const size_t numGroups = size_t(t.numGroups);
     if (t.subWalks == kWalkParts && numGroups <= size_t(16) * smCount)
         finishKernel<true><<<unsigned(std::min(numGroups, size_t(8) * smCount)), kFinishThreads, 0, s>>>(t, sink);

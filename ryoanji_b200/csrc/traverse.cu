@@ -350,9 +350,9 @@ __host__ __device__ constexpr int m2pBatch()
     return Nodes::kDipole || kImages ? kWarp : 2 * kWarp;
 }
 
-/*! evaluate @p count (<= m2pBatch) pending cells from the @p first on. With kImages the cells belong to several replicas
- *  of a periodic box and every cell's shift is staged too: a pair's distance is (target + shift) - cell, as where the
- *  targets are moved. */
+/*! evaluate @p count (<= m2pBatch) pending cells from the @p first on. With kImages the cells belong to several
+ *  replicas of a periodic box and every cell's shift is staged too: a pair's distance is (target + shift) - cell, as
+ *  where the targets are moved. */
 template<bool kImages = false, class Nodes>
 __device__ __forceinline__ void evalM2P(WarpSmem& S, int first, int count, const Nodes& nodes, const TargetState& T,
                                         const float* boxL = nullptr)
@@ -1075,7 +1075,8 @@ static void launchTyped(const TraverseLaunch& t, const Nodes& nodes, const Targe
     {
         auto kernel       = traverseKernel<Nodes, Targets, Sources>;
         const size_t smem = stack + sizeof(WarpSmem) * kTravWarps;
-        kernel<<<residentBlocks(kernel, smem, size_t(t.numGroups), smCount), kTravThreads, smem, s>>>(t, nodes, tgt, src);
+        kernel<<<residentBlocks(kernel, smem, size_t(t.numGroups), smCount), kTravThreads, smem, s>>>(t, nodes, tgt,
+                                                                                                      src);
         RYO_LAUNCH_CHECK();
         return;
     }

@@ -18,11 +18,11 @@
  *
  * As in float, launches of few groups go through interaction lists (lists.cuh) and larger ones through the fused
  * kernel. The list evaluation is bound by the FP64 pipe (13 operations, 26 cycles, per direct pair and sub-core; the
- * pipe is 70% busy) and the latency of its chains beside the conversions around rsqrt: it leaves the softening's maximum out
- * where a batch lies beyond it, and runs four sources of two targets at once. The step flow of 120,001 Plummer bodies,
- * everything double: 2.3 ms per pass, against 6.3 ms with the fused kernel (whose time is its longest group's); 250,000
- * bodies of a cube, float masses: 2.47 against 2.75 ms. Its evaluation takes 1.30 and 1.44 ms (two sources at once 1.32
- * and 1.53 ms, five blocks per SM 1.33 and 1.52 ms).
+ * pipe is 70% busy) and the latency of its chains beside the conversions around rsqrt: it leaves the softening's
+ * maximum out where a batch lies beyond it, and runs four sources of two targets at once. The step flow of 120,001
+ * Plummer bodies, everything double: 2.3 ms per pass, against 6.3 ms with the fused kernel (whose time is its longest
+ * group's); 250,000 bodies of a cube, float masses: 2.47 against 2.75 ms. Its evaluation takes 1.30 and 1.44 ms (two
+ * sources at once 1.32 and 1.53 ms, five blocks per SM 1.33 and 1.52 ms).
  */
 #include "lists.cuh"
 

@@ -1,5 +1,5 @@
-"""Leaf construction around the sizes where its scans and its sizing change: tiles of 4,096 values, four tiles scanned by
-one block, blocks of 256 keys, and 2^18 keys."""
+"""Leaf construction around the sizes where its scans and its sizing change: tiles of 4,096 values, four tiles scanned
+by one block, blocks of 256 keys, and 2^18 keys."""
 import numpy as np
 import pytest
 
