@@ -19,10 +19,11 @@
  * As in float, launches of few groups go through interaction lists (lists.cuh) and larger ones through the fused
  * kernel. The list evaluation is bound by the FP64 pipe (13 operations, 26 cycles, per direct pair and sub-core; the
  * pipe is 70% busy) and the latency of its chains beside the conversions around rsqrt: it leaves the softening's
- * maximum out where a batch lies beyond it, and runs four sources of two targets at once. The step flow of 120,001
- * Plummer bodies, everything double: 2.3 ms per pass, against 6.3 ms with the fused kernel (whose time is its longest
- * group's); 250,000 bodies of a cube, float masses: 2.47 against 2.75 ms. Its evaluation takes 1.30 and 1.44 ms (two
- * sources at once 1.32 and 1.53 ms, five blocks per SM 1.33 and 1.52 ms).
+ * maximum out where a batch lies beyond it, runs four sources of two targets at once, and reads staged cells 16 bytes
+ * at a time. The step flow of 120,001 Plummer bodies, everything double: 2.3 ms per pass, against 6.3 ms with the
+ * fused kernel (whose time is its longest group's); 250,000 bodies of a cube, float masses: 2.44 against 2.80 ms. Its
+ * evaluation takes 1.26 and 1.39 ms (two sources at once 1.32 and 1.53 ms, five blocks per SM 1.33 and 1.52 ms, cells
+ * read 8 bytes at a time from stages that share their banks 1.28 and 1.44 ms).
  */
 #include "lists.cuh"
 
@@ -33,7 +34,8 @@ constexpr int kT64Warps   = 4;
 constexpr int kT64Threads = kT64Warps * kWarp;
 constexpr int kT64M2PCap  = 2 * kWarp; // pending approximated cells (evaluated in rounds of 32)
 constexpr int kT64LeafCap = 2 * kWarp; // pending direct leaves (evaluated when more than 32 are pending)
-constexpr int kT64Stride  = 16;        // staged doubles per source: x, y, z, then 12 multipole values or m, h
+constexpr int kT64Stride  = 18;        // staged doubles per source: x, y, z, then 12 multipole values or m, h; 16 would
+                                       // put every source in the same banks
 constexpr int kT64Root    = -2;        // stack marker of a single-node tree
 
 struct WarpSmem64
@@ -454,7 +456,7 @@ struct Targets64
 
 struct EvalSmem64
 {
-    double stage[kWarp * kT64Stride];
+    alignas(16) double stage[kWarp * kT64Stride];
     int2 leaves[kWarp];
     int leafScan[kWarp];
 };
@@ -588,7 +590,13 @@ __global__ void __launch_bounds__(kTravThreads, 4) evalKernel64(TraverseLaunch P
                     __syncwarp();
                     for (int j = 0; j < count; ++j)
                     {
-                        const double* s = S.stage + j * kT64Stride;
+                        double s[14];
+#pragma unroll
+                        for (int k = 0; k < (kDipole ? 14 : 10); k += 2)
+                        {
+                            const double2 v = *reinterpret_cast<const double2*>(S.stage + j * kT64Stride + k);
+                            s[k] = v.x, s[k + 1] = v.y;
+                        }
 #pragma unroll
                         for (int t = 0; t < 2; ++t)
                             m2p64<kDipole>(acc[t], tx[t], ty[t], tz[t], s);
