@@ -631,13 +631,12 @@ void traverseLists(ryo_ctx* ctx, TraverseLaunch t, const uint32_t* list, uint32_
     RYO_CUDA(cudaMemsetAsync(t.groupState, 0, 3 * sizeof(uint32_t) * size_t(numGroups), s));
     uint32_t* unserved[2] = {ctx->scratch<uint32_t>("trav.unservedA", count, s),
                              ctx->scratch<uint32_t>("trav.unservedB", count, s)};
-    uint32_t chunk         = count; // groups per launch
-    const size_t perTarget = t.precision == kPrecisionF32 ? 1 : 2; // float4 per target's sums
+    uint32_t chunk = count; // groups per launch
     for (int flip = 0;; flip ^= 1)
     {
         t.items      = ctx->scratch<ListItem>("trav.items", t.itemCapacity, s);
         t.lists      = ctx->scratch<uint32_t>("trav.lists", size_t(t.itemCapacity) * t.itemWords, s);
-        t.partials   = ctx->scratch<float4>("trav.partials", size_t(t.itemCapacity) * 2 * kWarp * perTarget, s);
+        t.partials   = ctx->scratch<double4>("trav.partials", size_t(t.itemCapacity) * 2 * kWarp, s);
         uint32_t left = 0;
         for (uint32_t first = 0; first < count; first += chunk)
         {

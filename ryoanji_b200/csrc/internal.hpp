@@ -394,7 +394,7 @@ struct TraverseLaunch
     const uint32_t* groupList;
     ListItem* items;
     uint32_t* lists;
-    float4* partials;       // (phi, ax, ay, az) of an item's 64 targets; doubles for double coordinates
+    double4* partials;      // (phi, ax, ay, az) of an item's 64 targets
     uint32_t itemCapacity, itemWords;
     unsigned itemCost;
     int* taskLast;          // per part of a walk: its last item, -1 if its list is empty

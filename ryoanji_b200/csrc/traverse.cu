@@ -1040,14 +1040,25 @@ __global__ void __launch_bounds__(kTravThreads, kEvalBlocks)
                 }
             }
         }
-        const ListSums r = readSums(S);
         __syncwarp();
-        if (item.only) storeGroup(P, tgt, r, b, e, F.sys);
+        if (item.only) storeGroup(P, tgt, readSums(S), b, e, F.sys);
         else
         {
-            float4* out       = P.partials + size_t(it) * (2 * kWarp);
-            out[lane]         = make_float4(r.phi[0], r.x[0], r.y[0], r.z[0]);
-            out[kWarp + lane] = make_float4(r.phi[1], r.x[1], r.y[1], r.z[1]);
+            // with its compensation, so that a group's sum is rounded to float once, behind its last item
+            double v[4][2];
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+            {
+                float sum[2], comp[2];
+                upk(S.sums[0][k][lane], sum[0], sum[1]);
+                upk(S.sums[1][k][lane], comp[0], comp[1]);
+#pragma unroll
+                for (int t = 0; t < 2; ++t)
+                    v[k][t] = double(sum[t]) - double(comp[t]);
+            }
+            double4* out      = P.partials + size_t(it) * (2 * kWarp);
+            out[lane]         = make_double4(-v[0][0], v[1][0], v[2][0], v[3][0]);
+            out[kWarp + lane] = make_double4(-v[0][1], v[1][1], v[2][1], v[3][1]);
         }
     }
 }
@@ -1057,7 +1068,7 @@ template<class Targets>
 struct FloatSink
 {
     Targets tgt;
-    __device__ __forceinline__ float4 part(const TraverseLaunch& P, size_t i) const { return P.partials[i]; }
+    __device__ __forceinline__ double4 part(const TraverseLaunch& P, size_t i) const { return P.partials[i]; }
     __device__ __forceinline__ double store(const TraverseLaunch& P, int idx, const double s[4]) const
     {
         const float phi = float(s[0]), mi = tgt.scalar(idx);

@@ -680,7 +680,7 @@ __global__ void __launch_bounds__(kTravThreads, 4) evalKernel64(TraverseLaunch P
         }
         if (!item.only)
         {
-            double4* out = reinterpret_cast<double4*>(P.partials) + size_t(it) * (2 * kWarp);
+            double4* out = P.partials + size_t(it) * (2 * kWarp);
 #pragma unroll
             for (int t = 0; t < 2; ++t)
                 out[t * kWarp + lane] = make_double4(acc[t].phi, acc[t].x, acc[t].y, acc[t].z);
@@ -703,10 +703,7 @@ template<class Th, class Tm, class Ta, class Tmp>
 struct DoubleSink
 {
     Trav64<Th, Tm, Ta, Tmp> A;
-    __device__ __forceinline__ double4 part(const TraverseLaunch& P, size_t i) const
-    {
-        return reinterpret_cast<const double4*>(P.partials)[i];
-    }
+    __device__ __forceinline__ double4 part(const TraverseLaunch& P, size_t i) const { return P.partials[i]; }
     __device__ __forceinline__ double store(const TraverseLaunch& P, int idx, const double s[4]) const
     {
         return storeResult64(P, A, idx, Acc64{s[0], s[1], s[2], s[3]});
