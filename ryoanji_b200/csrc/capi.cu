@@ -545,17 +545,20 @@ extern "C" uint32_t ryo_stack_size(uint32_t) { return 0; }
 namespace
 {
 
-__global__ void splitGroupsKernel(const uint32_t* failed, uint32_t numFailed, const uint32_t* starts,
-                                  const uint32_t* ends, const uint32_t* sys, uint32_t* newStart, uint32_t* newEnd,
-                                  uint32_t* newSys, unsigned int* unsplit, unsigned int* numNew)
+//! the failed groups of @p t as halves; a single target cannot be split and gets zeros where the traversal stores results
+__global__ void splitGroupsKernel(const __grid_constant__ TraverseLaunch t, uint32_t numFailed, uint32_t* newStart,
+                                  uint32_t* newEnd, uint32_t* newSys, unsigned int* unsplit, unsigned int* numNew)
 {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= numFailed) return;
-    uint32_t g = failed[i];
-    uint32_t a = starts[g], b = ends[g];
+    uint32_t g = t.failedGroups[i];
+    uint32_t a = t.groupStart[g], b = t.groupEnd[g];
     if (b - a < 2)
     {
         atomicAdd(unsplit, 1u);
+        if (!t.overwrite) return;
+        if (t.p) t.p[a] = 0.f;
+        t.ax[a] = t.ay[a] = t.az[a] = 0.f;
         return;
     }
     uint32_t mid  = a + (b - a) / 2;
@@ -564,7 +567,7 @@ __global__ void splitGroupsKernel(const uint32_t* failed, uint32_t numFailed, co
     newEnd[slot]       = mid;
     newStart[slot + 1] = mid;
     newEnd[slot + 1]   = b;
-    if (sys) newSys[slot] = newSys[slot + 1] = sys[g];
+    if (t.groupSys) newSys[slot] = newSys[slot + 1] = t.groupSys[g];
 }
 
 /*! groups up to which a traversal goes through interaction lists: walks first, then the evaluation of list pieces of
@@ -707,8 +710,7 @@ void runTraversal(ryo_ctx* ctx, TraverseLaunch t, cudaStream_t s, double* potent
                                        : nullptr;
         unsigned int* cnt = ctx->ctl->counters;
         RYO_CUDA(cudaMemsetAsync(cnt, 0, 2 * sizeof(unsigned int), s));
-        splitGroupsKernel<<<ceilDiv(numFailed, 256), 256, 0, s>>>(failed, numFailed, t.groupStart, t.groupEnd,
-                                                                   t.groupSys, nStart, nEnd, nSys, cnt + 1, cnt);
+        splitGroupsKernel<<<ceilDiv(numFailed, 256), 256, 0, s>>>(t, numFailed, nStart, nEnd, nSys, cnt + 1, cnt);
         RYO_LAUNCH_CHECK();
         unsigned int h[2];
         RYO_CUDA(cudaMemcpyAsync(h, cnt, sizeof(h), cudaMemcpyDeviceToHost, s));
