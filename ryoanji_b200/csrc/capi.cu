@@ -619,7 +619,10 @@ void traverseLists(ryo_ctx* ctx, TraverseLaunch t, const uint32_t* list, uint32_
     const uint32_t numGroups = uint32_t(t.numGroups);
     // a caller's stack capacity is for one walk of the whole tree
     t.subWalks  = (list || solveGroups <= kSubGroups) && ownStack ? 8 : 1;
-    t.walkEntries = ownStack ? 8 : 4; // two steps at once need more stack, which a caller may have sized for one
+    // only parts of a walk take two steps at once: it makes another walk, and the depth of a whole walk is the caller's
+    t.walkEntries   = t.subWalks > 1 ? 8 : 4;
+    t.stackCapacity = std::min(t.stackCapacity, kMaxStackCapacity);
+    t.walkCapacity  = t.subWalks > 1 ? kMaxPartCapacity : t.stackCapacity;
     const unsigned minCost = t.groupSys ? kMinItemCost : std::min(kMinItemCost, 2 * solveGroups);
     t.itemCost  = std::min(kMaxItemCost, std::max(minCost, solveGroups / 2));
     t.itemWords = t.subWalks > 1 ? 512 : 2048;

@@ -28,6 +28,7 @@ struct Control
     unsigned int heavyCount;   // groups queued for the interaction-list kernels
     unsigned int itemCount;    // items of the interaction lists, and the head of their queue
     unsigned int itemHead;
+    unsigned int depthHead;     // of the groups whose walk's depth is taken
     unsigned int unservedCount; // groups whose list did not fit into the pool
 };
 
@@ -334,6 +335,12 @@ struct alignas(16) ListItem
     uint32_t only;  // 1 if it is the group's only item
 };
 
+// Stack entries that no walk passes. What lies on the stack above the entries of one step descends from them, so every
+// step whose entries are still there has a lowest level above that of the one before: at most 21 steps, of 8 entries
+// for each one taken. That is 672 entries for steps that take four, and 1,344 for two steps at once.
+constexpr int kMaxStackCapacity = 1024;
+constexpr int kMaxPartCapacity  = 21 * 64;
+
 //! why a group was not evaluated: its walk overflowed the stack, or found no free slot
 constexpr uint32_t kGroupFailed   = 1;
 constexpr uint32_t kGroupUnserved = 2;
@@ -391,6 +398,7 @@ struct TraverseLaunch
     // items of itemWords words, closed past itemCost interactions
     uint32_t subWalks;
     int walkEntries;        // stack entries that a float list walk takes at once: 4, or 8 for two steps
+    int walkCapacity;       // stack entries of a list walk: stackCapacity, or what a part of a walk never passes
     const uint32_t* groupList;
     ListItem* items;
     uint32_t* lists;

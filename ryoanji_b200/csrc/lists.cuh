@@ -7,8 +7,10 @@
  *
  * What bounds it: the walk of many groups is bound by instruction issue and the L1 (a step of 32 cells takes about 170
  * instructions with the list's writing; 5% of the evaluation's time), that of few groups by the latency of its longest
- * part. Two steps' cells loaded at once: 2^20 Plummer bodies 398 -> 338 us, 60,001 bodies 132 -> 112 us. The lists take
- * 6-15 KB per group and stay in the L2 between the two kernels.
+ * part. The parts of a divided walk load two steps' cells at once: 60,001 Plummer bodies 132 -> 112 us. A whole walk
+ * does not, which costs it up to a fifth of its time (2^20 bodies 398 against 338 us, 1% of the solve): it is the walk
+ * whose depth the caller sees. Divided ones have theirs taken beside the evaluation (walkDepth), at 1 to 3% of a solve.
+ * The lists take 6-15 KB per group and stay in the L2 between the two kernels.
  */
 #pragma once
 
@@ -185,6 +187,101 @@ struct ListWriter
     }
 };
 
+//! centre and half extent of the bounding box of group @p g
+template<class R, class Targets>
+__device__ __forceinline__ void groupBox(const TraverseLaunch& P, const Targets& tgt, unsigned g, R tc[3], R ts[3])
+{
+    using F     = Fp<R>;
+    const int b = int(P.groupStart[g]), e = int(P.groupEnd[g]);
+    R u[3], v[3];
+    tgt.position(min(b + int(laneId()), e - 1), u);
+    tgt.position(min(b + kWarp + int(laneId()), e - 1), v);
+#pragma unroll
+    for (int d = 0; d < 3; ++d)
+    {
+        const R l = warpMin(fmin(u[d], v[d])), h = warpMax(fmax(u[d], v[d]));
+        tc[d]     = F::mul(F::add(h, l), R(0.5));
+        ts[d]     = F::mul(F::sub(h, l), R(0.5));
+    }
+}
+
+/*! the most entries that the undivided walk of group @p g holds, four taken per step: the depth that a caller's stack
+ *  capacity bounds and that the statistics report. The parts of a divided walk have other depths, since each starts
+ *  lower and takes two steps at once. False if the walk passes P.stackCapacity. */
+template<class Nodes, class Targets>
+__device__ __forceinline__ bool walkDepth(const TraverseLaunch& P, const Nodes& nodes, const Targets& tgt, unsigned g,
+                                          int* stack, int& maxStack)
+{
+    const int lane    = laneId();
+    const unsigned lt = lanemaskLt();
+    using R = typename Nodes::Real;
+    using F = Fp<R>;
+    R tc[3], ts[3];
+    groupBox(P, tgt, g, tc, ts);
+    GroupFrame<R> G;
+    G.set(P, g);
+    maxStack = 0;
+    for (int iz = -G.shells; iz <= G.shells; ++iz)
+        for (int iy = -G.shells; iy <= G.shells; ++iy)
+            for (int ix = -G.shells; ix <= G.shells; ++ix)
+            {
+                const R sh[3] = {F::mul(R(ix), G.boxL[0]), F::mul(R(iy), G.boxL[1]), F::mul(R(iz), G.boxL[2])};
+#pragma unroll
+                for (int d = 0; d < 3; ++d)
+                    tc[d] = F::add(tc[d], sh[d]);
+                int sp = 1;
+                __syncwarp();
+                if (lane == 0) stack[0] = G.rootEntry;
+                __syncwarp();
+                while (sp > 0)
+                {
+                    const int k     = min(4, sp), at = k - 4 + (lane >> 3);
+                    sp -= k;
+                    const int entry = at >= 0 ? stack[sp + at] : -1;
+                    int cell        = -1;
+                    if (entry <= kRootOnly) cell = (lane & 7) == 0 ? kRootOnly - entry : -1;
+                    else if (entry >= 0) cell = entry + (lane & 7);
+                    __syncwarp();
+                    typename Nodes::Center c = {};
+                    int4 link                = {};
+                    if (cell >= 0) nodes.load(cell, c, link);
+                    const bool split  = cell >= 0 && macFails(c, tc, ts) && link.x != 0;
+                    const unsigned bs = __ballot_sync(0xffffffffu, split);
+                    if (sp + __popc(bs) > P.stackCapacity) return false;
+                    if (split) stack[sp + __popc(bs & lt)] = link.x;
+                    sp += __popc(bs);
+                    maxStack = max(maxStack, sp);
+                    __syncwarp();
+                }
+#pragma unroll
+                for (int d = 0; d < 3; ++d)
+                    tc[d] = F::sub(tc[d], sh[d]);
+            }
+    return true;
+}
+
+/*! the depths of the launch's groups whose walks were divided, taken by the evaluation's warps before its items; a
+ *  group that passes the stack's capacity has failed. @p stack holds P.stackCapacity entries. */
+template<class Nodes, class Targets>
+__device__ __forceinline__ void depthTasks(const TraverseLaunch& P, const Nodes& nodes, const Targets& tgt, int* stack)
+{
+    while (true)
+    {
+        unsigned i = 0;
+        if (laneId() == 0) i = atomicAdd(&P.ctl->depthHead, 1u);
+        i = __shfl_sync(0xffffffffu, i, 0);
+        if (i >= unsigned(P.numGroups)) return;
+        const unsigned g = P.groupList ? P.groupList[i] : i;
+        int depth;
+        const bool ok = walkDepth(P, nodes, tgt, g, stack, depth);
+        __syncwarp();
+        if (laneId() != 0) continue;
+        atomicMax(&P.ctl->stats[kMaxStack], (unsigned long long)depth);
+        if (!ok && atomicCAS(&P.groupState[g], 0u, kGroupFailed) == 0u)
+            P.failedGroups[atomicAdd(&P.ctl->failedCount, 1u)] = g;
+    }
+}
+
 /*! walks the tree for one task and writes the interaction list to @p L: a group's whole walk, or part @p sub of
  *  P.subWalks parts. False if the walk overflowed the stack or was starved. */
 template<class Nodes, class Targets>
@@ -194,25 +291,13 @@ __device__ __forceinline__ bool walkTask(const TraverseLaunch& P, const Nodes& n
 {
     const int lane    = laneId();
     const unsigned lt = lanemaskLt();
-    const int b = int(P.groupStart[g]), e = int(P.groupEnd[g]);
     using R = typename Nodes::Real;
     using F = Fp<R>;
     // steps whose cells are loaded at once; in double a second one costs more registers than the latency is worth (the
     // walk of 120,001 Plummer bodies 88 -> 100 us)
     constexpr int kSteps = std::is_same_v<R, float> ? 2 : 1;
     R tc[3], ts[3];
-    {
-        R u[3], v[3];
-        tgt.position(min(b + lane, e - 1), u);
-        tgt.position(min(b + kWarp + lane, e - 1), v);
-#pragma unroll
-        for (int d = 0; d < 3; ++d)
-        {
-            const R l = warpMin(fmin(u[d], v[d])), h = warpMax(fmax(u[d], v[d]));
-            tc[d]     = F::mul(F::add(h, l), R(0.5));
-            ts[d]     = F::mul(F::sub(h, l), R(0.5));
-        }
-    }
+    groupBox(P, tgt, g, tc, ts);
     GroupFrame<R> G;
     G.set(P, g);
     // a part takes one child of the root, or in a periodic group every subWalks-th replica; a single-cell tree belongs
@@ -287,7 +372,7 @@ __device__ __forceinline__ bool walkTask(const TraverseLaunch& P, const Nodes& n
                         bool split  = close && isNode;
                         unsigned bs = __ballot_sync(0xffffffffu, split);
                         int nsplit  = __popc(bs);
-                        if (sp + nsplit > P.stackCapacity)
+                        if (sp + nsplit > P.walkCapacity)
                         {
                             overflow = true;
                             break;
@@ -366,7 +451,7 @@ __global__ void __launch_bounds__(kTravThreads) walkKernel(TraverseLaunch P, Nod
     extern __shared__ __align__(16) unsigned char smemRaw[];
     const int warp = threadIdx.x / kWarp, lane = laneId();
     WalkSmem& W    = reinterpret_cast<WalkSmem*>(smemRaw)[warp];
-    int* stack     = reinterpret_cast<int*>(smemRaw + sizeof(WalkSmem) * kTravWarps) + warp * P.stackCapacity;
+    int* stack     = reinterpret_cast<int*>(smemRaw + sizeof(WalkSmem) * kTravWarps) + warp * P.walkCapacity;
     const unsigned numTasks = unsigned(P.numGroups) * P.subWalks;
     while (true)
     {
@@ -383,7 +468,7 @@ __global__ void __launch_bounds__(kTravThreads) walkKernel(TraverseLaunch P, Nod
         __syncwarp();
         if (lane != 0) continue;
         P.taskLast[task] = L.item;
-        if (!L.starved) atomicMax(&P.ctl->stats[kMaxStack], (unsigned long long)maxStack);
+        if (!L.starved && P.subWalks == 1) atomicMax(&P.ctl->stats[kMaxStack], (unsigned long long)maxStack);
         if (!ok)
         {
             // nothing of this group is evaluated: it goes back to the host, to be walked again when the pool is free,
@@ -534,7 +619,7 @@ template<class Nodes, class Targets>
 void launchWalk(const TraverseLaunch& t, const Nodes& nodes, const Targets& tgt, int smCount, cudaStream_t s)
 {
     auto walk         = walkKernel<Nodes, Targets>;
-    const size_t smem = (sizeof(int) * size_t(t.stackCapacity) + sizeof(WalkSmem)) * kTravWarps;
+    const size_t smem = (sizeof(int) * size_t(t.walkCapacity) + sizeof(WalkSmem)) * kTravWarps;
     walk<<<residentBlocks(walk, smem, size_t(t.numGroups) * t.subWalks, smCount), kTravThreads, smem, s>>>(t, nodes,
                                                                                                           tgt);
     RYO_LAUNCH_CHECK();

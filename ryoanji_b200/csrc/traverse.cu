@@ -632,6 +632,7 @@ __global__ void resetTraversal(Control* ctl, int what)
     ctl->workCounter   = 0;
     ctl->itemCount     = 0;
     ctl->itemHead      = 0;
+    ctl->depthHead     = 0;
     ctl->unservedCount = 0;
     if (what == kTravLists) return;
     ctl->failedCount = 0;
@@ -928,8 +929,8 @@ __global__ void __launch_bounds__(kTravThreads, 5)
 }
 
 /*! evaluates the interaction lists. Warps take items from the queue; the sums of a group's only item are the group's
- *  results, others go to P.partials for finishKernel. */
-template<class Nodes, class Targets, class Sources>
+ *  results, others go to P.partials for finishKernel. With kParts, for divided walks, the groups' depths come first. */
+template<bool kParts, class Nodes, class Targets, class Sources>
 __global__ void __launch_bounds__(kTravThreads, kEvalBlocks)
     evalKernel(TraverseLaunch P, Nodes nodes, Targets tgt, Sources src)
 {
@@ -937,6 +938,8 @@ __global__ void __launch_bounds__(kTravThreads, kEvalBlocks)
     WarpSmem& S    = smem[threadIdx.x / kWarp];
     const int lane = laneId();
     const unsigned numItems = min(P.ctl->itemCount, P.itemCapacity);
+    static_assert(sizeof(S.stage) >= kMaxStackCapacity * sizeof(int));
+    if constexpr (kParts) depthTasks(P, nodes, tgt, reinterpret_cast<int*>(S.stage));
     while (true)
     {
         unsigned it = 0;
@@ -1041,7 +1044,7 @@ __global__ void __launch_bounds__(kTravThreads, kEvalBlocks)
             }
         }
         __syncwarp();
-        if (item.only) storeGroup(P, tgt, readSums(S), b, e, F.sys);
+        if (!kParts && item.only) storeGroup(P, tgt, readSums(S), b, e, F.sys);
         else
         {
             // with its compensation, so that a group's sum is rounded to float once, behind its last item
@@ -1092,7 +1095,7 @@ static void launchTyped(const TraverseLaunch& t, const Nodes& nodes, const Targe
         return;
     }
     launchWalk(t, nodes, tgt, smCount, s);
-    auto eval = evalKernel<Nodes, Targets, Sources>;
+    auto eval = t.subWalks > 1 ? evalKernel<true, Nodes, Targets, Sources> : evalKernel<false, Nodes, Targets, Sources>;
     eval<<<residentBlocks(eval, 0, size_t(t.itemCapacity), smCount), kTravThreads, 0, s>>>(t, nodes, tgt, src);
     RYO_LAUNCH_CHECK();
     launchFinish(t, FloatSink<Targets>{tgt}, smCount, s);

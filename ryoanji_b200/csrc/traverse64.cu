@@ -493,6 +493,10 @@ __global__ void __launch_bounds__(kTravThreads, 4) evalKernel64(TraverseLaunch P
     EvalSmem64& S  = smem[threadIdx.x / kWarp];
     const int lane = laneId();
     const unsigned numItems = min(P.ctl->itemCount, P.itemCapacity);
+    static_assert(sizeof(S.stage) >= kMaxStackCapacity * sizeof(int));
+    if (P.subWalks > 1)
+        depthTasks(P, Nodes64{A.centers, P.childOffsets, P.internalToLeaf, P.layout}, Targets64{A.xt, A.yt, A.zt},
+                   reinterpret_cast<int*>(S.stage));
     while (true)
     {
         unsigned it = 0;
