@@ -614,11 +614,10 @@ void readControl(ryo_ctx* ctx, Control& c, cudaStream_t s)
  *  overflowed the stack. Lists are cut by the solve's group count and the walk alone, so a group's sums do not depend
  *  on the launch or pass that it falls in. */
 void traverseLists(ryo_ctx* ctx, TraverseLaunch t, const uint32_t* list, uint32_t count, uint32_t solveGroups,
-                   bool ownStack, Control& c, cudaStream_t s)
+                   Control& c, cudaStream_t s)
 {
     const uint32_t numGroups = uint32_t(t.numGroups);
-    // a caller's stack capacity is for one walk of the whole tree
-    t.subWalks  = (list || solveGroups <= kSubGroups) && ownStack ? 8 : 1;
+    t.subWalks  = list || solveGroups <= kSubGroups ? 8 : 1;
     // only parts of a walk take two steps at once: it makes another walk, and the depth of a whole walk is the caller's
     t.walkEntries   = t.subWalks > 1 ? 8 : 4;
     t.stackCapacity = std::min(t.stackCapacity, kMaxStackCapacity);
@@ -670,8 +669,7 @@ void runTraversal(ryo_ctx* ctx, TraverseLaunch t, cudaStream_t s, double* potent
 {
     const uint32_t numGroups = uint32_t(t.numGroups);
     t.ctl                    = ctx->ctl;
-    const bool ownStack      = t.stackCapacity <= 0;
-    if (ownStack) t.stackCapacity = 512; // the deepest walks measured use about 110 entries
+    if (t.stackCapacity <= 0) t.stackCapacity = 512; // the deepest walks measured use about 110 entries
     launchTraversalReset(ctx->ctl, kTravAll, s);
     ctx->retries          = 0;
     bool unsplittable     = false;
@@ -687,7 +685,7 @@ void runTraversal(ryo_ctx* ctx, TraverseLaunch t, cudaStream_t s, double* potent
         if (pass > 0) launchTraversalReset(ctx->ctl, kTravPass, s);
         ++pass;
         if (solveGroups <= kListGroups)
-            traverseLists(ctx, t, nullptr, uint32_t(t.numGroups), solveGroups, ownStack, hc, s);
+            traverseLists(ctx, t, nullptr, uint32_t(t.numGroups), solveGroups, hc, s);
         else
         {
             t.heavyGroups   = ctx->scratch<uint32_t>("trav.heavy", std::max(t.numGroups, 1), s);
@@ -699,7 +697,7 @@ void runTraversal(ryo_ctx* ctx, TraverseLaunch t, cudaStream_t s, double* potent
             {
                 // groups too long for one warp go through lists, whose pieces all warps share
                 launchTraversalReset(ctx->ctl, kTravLists, s);
-                traverseLists(ctx, t, t.heavyGroups, hc.heavyCount, solveGroups, ownStack, hc, s);
+                traverseLists(ctx, t, t.heavyGroups, hc.heavyCount, solveGroups, hc, s);
             }
         }
         unsigned int numFailed = hc.failedCount;

@@ -1,5 +1,5 @@
 """The stack depth that a traversal reports is the one a caller's stack capacity is compared with: that capacity fits
-without a split, one entry less does not."""
+without a split, one entry less does not. Any capacity that fits gives the default's results, bit for bit."""
 import numpy as np
 import pytest
 import torch
@@ -48,6 +48,30 @@ def test_depth_is_the_capacity_that_fits(kind, n, group):
     _tight(run)
 
 
+# as above, from a single leaf on, and with signed expansions
+@pytest.mark.parametrize("kind,n,mdq", [("plummer", 40, False), ("plummer", 1000, False), ("plummer", 60001, False),
+                                        ("periodic", 20011, False), ("gauss", 100003, True), ("plummer", 500009, False),
+                                        ("plummer", 3200007, False)])
+def test_capacities_that_fit_give_the_same_bits(kind, n, mdq):
+    import ryoanji_b200 as ryo
+    from ryoanji_b200 import datasets as ds
+    p = (ds.plummer(n, seed=n, velocities=False) if kind == "plummer" else
+         ds.periodic_box(n, seed=n, eps=0.002) if kind == "periodic" else ds.gaussian(n, seed=n, sigma=0.3))
+    box = ryo.Box(*p.box, boundary=(ryo.BOUNDARY_PERIODIC,) * 3) if kind == "periodic" else None
+    ctx = ryo.Context()
+
+    def run(capacity):
+        out = torch.empty(4, n, device="cuda")
+        r = ryo.solve(*(dev(a) for a in (p.x, p.y, p.z, p.m, p.h)), *out,
+                      ryo.SolveParams(theta=0.5, box=box, multipole="mdq" if mdq else "quadrupole",
+                                      stack_capacity=capacity), ctx=ctx)
+        return r, out
+    r, base = run(0)
+    for capacity in (max(r.max_stack, 1), 512, 1024, 5000):
+        q, out = run(capacity)
+        assert torch.equal(out, base) and q.max_stack == r.max_stack and q.retries == 0
+
+
 @pytest.mark.parametrize("real", [torch.float64, torch.float32])
 @pytest.mark.parametrize("n", [3000, 60001])
 def test_depth_of_double_traversals(real, n):
@@ -73,5 +97,10 @@ def test_depth_of_double_traversals(real, n):
         ryo.traverse(groups, 1, x, y, z, m, h, x, y, z, m, h, tb.childOffsets(), tb.internalToLeaf(), tb.layout(),
                      centers, mp, 1.0, 0, box.lengths, *out, stack_capacity=capacity)
         s = ryo.read_bh_stats()
+        results.append(out)
         return s[4], ryo.read_traversal_retries(), s[:4]
+    results = []
     _tight(run)
+    run(512)
+    for k in (1, -1):  # the depth's own capacity, and the default's size given
+        assert all(torch.equal(a, b) for a, b in zip(results[0], results[k]))
