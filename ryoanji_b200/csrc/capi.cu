@@ -574,6 +574,11 @@ __global__ void splitGroupsKernel(const __grid_constant__ TraverseLaunch t, uint
  *  similar cost by all warps. Larger ones keep the GPU busy with a group per warp, which saves the lists' traffic. */
 constexpr uint32_t kListGroups  = 49152;
 constexpr uint32_t kSubGroups   = 6000;  // groups up to which every list walk is split into eight parts
+// stack capacities below which divided walks have their depths taken before them. Open and periodic solves hold up to
+// about 110 entries, so below that groups may fail, whose lists and sums would be for nothing (250,000 bodies of a
+// cube, a capacity of 6 entries: 16.7 -> 4.9 ms); where all fit, it costs the longest walk's time (60,001 Plummer
+// bodies, 72 entries: 0.80 -> 0.87 ms)
+constexpr int kDepthFirst = 128;
 constexpr size_t kListBytes     = size_t(512) << 20; // of list items
 // interactions of an item: half the groups' number, at least 1024 (16 evaluation batches), below 512 groups twice their
 // number, so that the items of the smallest solves still number as many as the GPU has warps: 1,000 bodies 303 -> 267
@@ -621,6 +626,7 @@ void traverseLists(ryo_ctx* ctx, TraverseLaunch t, const uint32_t* list, uint32_
     // only parts of a walk take two steps at once: it makes another walk, and the depth of a whole walk is the caller's
     t.walkEntries   = t.subWalks > 1 ? 8 : 4;
     t.stackCapacity = std::min(t.stackCapacity, kMaxStackCapacity);
+    t.depthFirst    = t.subWalks > 1 && t.stackCapacity < kDepthFirst;
     t.walkCapacity  = t.subWalks > 1 ? kMaxPartCapacity : t.stackCapacity;
     const unsigned minCost = t.groupSys ? kMinItemCost : std::min(kMinItemCost, 2 * solveGroups);
     t.itemCost  = std::min(kMaxItemCost, std::max(minCost, solveGroups / 2));

@@ -398,6 +398,7 @@ struct TraverseLaunch
     // items of itemWords words, closed past itemCost interactions
     uint32_t subWalks;
     int walkEntries;        // stack entries that a float list walk takes at once: 4, or 8 for two steps
+    int depthFirst;         // divided walks: 1 takes the groups' depths before the walks, 0 in the evaluation
     int walkCapacity;       // stack entries of a list walk: stackCapacity, or what a part of a walk never passes
     const uint32_t* groupList;
     ListItem* items;

@@ -282,6 +282,14 @@ __device__ __forceinline__ void depthTasks(const TraverseLaunch& P, const Nodes&
     }
 }
 
+//! the depths before any walk, for a capacity that some groups may pass: they are neither walked nor evaluated
+template<class Nodes, class Targets>
+__global__ void __launch_bounds__(kTravThreads) depthKernel(TraverseLaunch P, Nodes nodes, Targets tgt)
+{
+    extern __shared__ __align__(16) unsigned char smemRaw[];
+    depthTasks(P, nodes, tgt, reinterpret_cast<int*>(smemRaw) + threadIdx.x / kWarp * P.stackCapacity);
+}
+
 /*! walks the tree for one task and writes the interaction list to @p L: a group's whole walk, or part @p sub of
  *  P.subWalks parts. False if the walk overflowed the stack or was starved. */
 template<class Nodes, class Targets>
@@ -461,6 +469,7 @@ __global__ void __launch_bounds__(kTravThreads) walkKernel(TraverseLaunch P, Nod
         if (task >= numTasks) return;
         const unsigned sub = task % P.subWalks;
         const unsigned g   = P.groupList ? P.groupList[task / P.subWalks] : task / P.subWalks;
+        if (P.depthFirst && P.groupState[g] != 0u) continue;
         ListWriter L;
         unsigned nM2P, nP2P;
         int maxStack;
@@ -618,6 +627,13 @@ unsigned residentBlocks(Kernel kernel, size_t smem, size_t warps, int smCount)
 template<class Nodes, class Targets>
 void launchWalk(const TraverseLaunch& t, const Nodes& nodes, const Targets& tgt, int smCount, cudaStream_t s)
 {
+    if (t.depthFirst)
+    {
+        auto depth        = depthKernel<Nodes, Targets>;
+        const size_t smem = sizeof(int) * size_t(t.stackCapacity) * kTravWarps;
+        depth<<<residentBlocks(depth, smem, size_t(t.numGroups), smCount), kTravThreads, smem, s>>>(t, nodes, tgt);
+        RYO_LAUNCH_CHECK();
+    }
     auto walk         = walkKernel<Nodes, Targets>;
     const size_t smem = (sizeof(int) * size_t(t.walkCapacity) + sizeof(WalkSmem)) * kTravWarps;
     walk<<<residentBlocks(walk, smem, size_t(t.numGroups) * t.subWalks, smCount), kTravThreads, smem, s>>>(t, nodes,

@@ -72,6 +72,27 @@ def test_capacities_that_fit_give_the_same_bits(kind, n, mdq):
         assert torch.equal(out, base) and q.max_stack == r.max_stack and q.retries == 0
 
 
+@pytest.mark.parametrize("capacity", [20, 40])
+def test_capacity_that_most_groups_pass(capacity):
+    """groups split until they fit; the expansions' error at theta 0.5 stays"""
+    import ryoanji_b200 as ryo
+    from ryoanji_b200 import datasets as ds
+    n = 20011
+    p = ds.plummer(n, seed=n, velocities=False)
+    t, out = [dev(a) for a in (p.x, p.y, p.z, p.m, p.h)], torch.full((4, n), float("nan"), device="cuda")
+    ctx = ryo.Context()
+    try:
+        ryo.solve(*t, *out, ryo.SolveParams(theta=0.5, bucket_size=32, stack_capacity=capacity), ctx=ctx)
+    except ryo.RyoError as e:
+        assert e.status == 4  # a target of its own passes the capacity too, and gets zeros
+    assert ryo.read_bh_stats(ctx)[4] <= capacity and ryo.read_traversal_retries(ctx) > 50
+    a = torch.stack(ryo.direct_targets_f64(torch.arange(n, device="cuda"), *t)[1:])
+    done = out[0] != 0
+    assert done.any()
+    err = ((out[1:].double() - a).norm(dim=0) / a.norm(dim=0))[done].cpu().numpy()
+    assert np.percentile(err, 99) < 1e-3 and np.median(err) < 2e-4
+
+
 @pytest.mark.parametrize("real", [torch.float64, torch.float32])
 @pytest.mark.parametrize("n", [3000, 60001])
 def test_depth_of_double_traversals(real, n):
