@@ -511,9 +511,10 @@ constexpr int kFinishThreads = 256;
 constexpr int kWalkParts     = kFinishThreads / kWarp; // parts of a divided walk
 
 /*! every group of the launch: interaction counts and statistics, and the results of the groups whose list became items
- *  (or is empty): the items' sums added in FP64 in a fixed order. @p sink reads the items' sums and stores a target's
- *  results, returning its m phi. Bound by the latency of the chains of items: a warp follows those of a group's parts
- *  one after the other, with kParts the warps of a block at once. */
+ *  (or is empty): the items' sums added in FP64, each part of the walk from its last item to its first, then the parts.
+ *  @p sink reads the items' sums and stores a target's results, returning its m phi. Bound by the latency of the chains
+ *  of items: a warp follows those of a group's parts one after the other, with kParts the warps of a block at once. The
+ *  order of the additions is the same, so a launch may take either. */
 template<bool kParts, class Sink>
 __global__ void __launch_bounds__(kFinishThreads) finishKernel(TraverseLaunch P, Sink sink)
 {
@@ -545,18 +546,24 @@ __global__ void __launch_bounds__(kFinishThreads) finishKernel(TraverseLaunch P,
         }
         for (unsigned sub = kParts ? warp : 0; sub < P.subWalks; sub += kParts ? kWalkParts : 1)
         {
+            double part[2][4] = {};
             for (int it = P.taskLast[i * P.subWalks + sub]; it >= 0; it = P.items[it].prev)
             {
 #pragma unroll
                 for (int t = 0; t < 2; ++t)
                 {
                     const auto v = sink.part(P, size_t(it) * (2 * kWarp) + t * kWarp + lane);
-                    sum[t][0] += v.x;
-                    sum[t][1] += v.y;
-                    sum[t][2] += v.z;
-                    sum[t][3] += v.w;
+                    part[t][0] += v.x;
+                    part[t][1] += v.y;
+                    part[t][2] += v.z;
+                    part[t][3] += v.w;
                 }
             }
+#pragma unroll
+            for (int t = 0; t < 2; ++t)
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+                    sum[t][k] += part[t][k];
         }
         if constexpr (kParts)
         {

@@ -45,3 +45,47 @@ def test_items_are_added_without_rounding():
         ulp = np.spacing(np.abs(a).astype(np.float32)).astype(np.float64)
         assert np.abs(a - exact).max() > 0  # not every result fits into a float
         assert (np.abs(a - exact) / ulp).max() <= 0.5
+
+
+def test_host_launches_add_in_the_order_of_the_device_solve():
+    """pageable outputs: eight launches of 375 groups each, whose items are added by a block per group; the device
+    solve's 3,000 groups by a warp each. The heavy octants' sums, of some hundreds, nearly cancel in the results, and two
+    octants' masses are so small that the others' sums leave out some of their bits in float64."""
+    import ryoanji_b200 as ryo
+    rng = np.random.default_rng(5)
+    n = 24000
+    pos = rng.uniform(-0.25, 0.25, (n, 3)).astype(np.float32)
+    m = np.where((pos > 0).sum(1) % 2 == 0, 1.0, -1.0) * rng.uniform(0.5, 1.0, n)
+    light = (pos[:, 0] > 0) & (pos[:, 1] > 0)
+    heavy = np.concatenate([np.ones((n, 1)), pos], 1)[~light].astype(np.float64)
+    basis = np.linalg.qr(heavy)[0]
+    m[~light] -= basis @ (basis.T @ m[~light])  # the heavy bodies have neither a total mass nor a dipole
+    m[light] *= 2.0 ** -30
+    m = m.astype(np.float32)
+    bodies = [torch.from_numpy(np.ascontiguousarray(v)) for v in (*pos.T, m, np.full(n, 0.5, np.float32))]
+    params = ryo.SolveParams(theta=0.01, bucket_size=32, group_size=8, box=ryo.Box.cube(-0.25, 0.25))
+    ctx = ryo.Context()
+    host = [torch.empty(n) for _ in range(4)]
+    ryo.solve_host(*bodies, *host, params=params, ctx=ctx)
+    dev = [torch.empty(n, device="cuda") for _ in range(4)]
+    r = ryo.solve(*(v.cuda() for v in bodies), *dev, params, ctx=ctx)
+    assert r.num_groups == 3000
+    assert max(v.abs().median() for v in host[1:]) < 1e-2  # the parts' sums do cancel
+    for a, b in zip(host, dev):
+        assert torch.equal(a, b.cpu())
+
+
+def test_host_solve_of_a_clustered_set_equals_the_device_solve():
+    import ryoanji_b200 as ryo
+    from ryoanji_b200 import datasets as ds
+    n = 300007
+    p = ds.plummer(n, seed=9, velocities=False)
+    bodies = [torch.from_numpy(a) for a in (p.x, p.y, p.z, p.m, p.h)]
+    ctx = ryo.Context()
+    host = [torch.empty(n) for _ in range(4)]
+    rh = ryo.solve_host(*bodies, *host, params=ryo.SolveParams(theta=0.5), ctx=ctx)
+    dev = [torch.empty(n, device="cuda") for _ in range(4)]
+    rd = ryo.solve(*(v.cuda() for v in bodies), *dev, ryo.SolveParams(theta=0.5), ctx=ctx)
+    assert 2369 <= rd.num_groups <= 6000 and rh.max_stack == rd.max_stack
+    for a, b in zip(host, dev):
+        assert torch.equal(a, b.cpu())
