@@ -128,13 +128,14 @@ __global__ void ewaldKernel(const __grid_constant__ EwaldKernelParams<R> E, cons
                             const Tc* __restrict__ y, const Tc* __restrict__ z, const Tm* __restrict__ m, float G,
                             Ta* ugrav, Ta* ax, Ta* ay, Ta* az, double* potential)
 {
-    const unsigned warpGlobal = (blockIdx.x * blockDim.x + threadIdx.x) / kWarp;
-    const int lane            = laneId();
-    double upot               = 0.0;
+    // from 2^26 groups on the threads' numbers pass 32 bits
+    const size_t warpGlobal = (size_t(blockIdx.x) * blockDim.x + threadIdx.x) / kWarp;
+    const int lane          = laneId();
+    double upot             = 0.0;
     if (warpGlobal / 2 < numGroups)
     {
         uint32_t b = groupStart[warpGlobal / 2], e = groupEnd[warpGlobal / 2];
-        for (uint32_t i = b + (warpGlobal & 1) * kWarp + lane; i < e; i += 2 * kWarp)
+        for (size_t i = b + (warpGlobal & 1) * kWarp + lane; i < e; i += 2 * kWarp)
         {
             R pos[3]  = {R(x[i]), R(y[i]), R(z[i])};
             R acc[4]  = {E.k1 * E.mroot[0], R(0), R(0), R(0)};
