@@ -98,7 +98,7 @@ __global__ void __launch_bounds__(kDirectThreads) directKernel(size_t first, siz
             }
     if (t < last)
     {
-        p[t] += m[t] * acc[0];
+        if (p) p[t] += m[t] * acc[0];
         ax[t] += acc[1];
         ay[t] += acc[2];
         az[t] += acc[3];
