@@ -579,6 +579,9 @@ constexpr uint32_t kSubGroups   = 6000;  // groups up to which every list walk i
 // cube, a capacity of 6 entries: 16.7 -> 4.9 ms); where all fit, it costs the longest walk's time (60,001 Plummer
 // bodies, 72 entries: 0.80 -> 0.87 ms)
 constexpr int kDepthFirst = 128;
+// the largest stack capacities accepted, for float and double coordinates: four warps' stacks beside the fused kernels'
+// staging in 227 KB of shared memory. No walk needs more than kMaxStackCapacity, which all kernels have room for.
+constexpr int kMostCapacity = 12344, kMostCapacity64 = 13120;
 constexpr size_t kListBytes     = size_t(512) << 20; // of list items
 // interactions of an item: half the groups' number, at least 1024 (16 evaluation batches), below 512 groups twice their
 // number, so that the items of the smallest solves still number as many as the GPU has warps: 1,000 bodies 303 -> 267
@@ -625,7 +628,6 @@ void traverseLists(ryo_ctx* ctx, TraverseLaunch t, const uint32_t* list, uint32_
     t.subWalks  = list || solveGroups <= kSubGroups ? 8 : 1;
     // only parts of a walk take two steps at once: it makes another walk, and the depth of a whole walk is the caller's
     t.walkEntries   = t.subWalks > 1 ? 8 : 4;
-    t.stackCapacity = std::min(t.stackCapacity, kMaxStackCapacity);
     t.depthFirst    = t.subWalks > 1 && t.stackCapacity < kDepthFirst;
     t.walkCapacity  = t.subWalks > 1 ? kMaxPartCapacity : t.stackCapacity;
     const unsigned minCost = t.groupSys ? kMinItemCost : std::min(kMinItemCost, 2 * solveGroups);
@@ -676,6 +678,9 @@ void runTraversal(ryo_ctx* ctx, TraverseLaunch t, cudaStream_t s, double* potent
     const uint32_t numGroups = uint32_t(t.numGroups);
     t.ctl                    = ctx->ctl;
     if (t.stackCapacity <= 0) t.stackCapacity = 512; // the deepest walks measured use about 110 entries
+    const int most = t.precision == kPrecisionF32 ? kMostCapacity : kMostCapacity64;
+    if (numGroups > 0 && t.stackCapacity > most) throw CudaError{cudaErrorInvalidValue, "traversal: stack capacity"};
+    t.stackCapacity = std::min(t.stackCapacity, kMaxStackCapacity);
     launchTraversalReset(ctx->ctl, kTravAll, s);
     ctx->retries          = 0;
     bool unsplittable     = false;
