@@ -494,7 +494,11 @@ extern "C"
 
     /* x, y, z, m, h: in any order on entry, SFC-sorted on return; vx, vy, vz (may be NULL) are permuted along;
      * p, ax, ay, az are overwritten with the potential (G m phi) and acceleration in sorted order; order (may be
-     * NULL) receives the original index of each sorted body. stats (host, may be NULL). */
+     * NULL) receives the original index of each sorted body. stats (host, may be NULL).
+     * Device scratch: about 130 bytes per body, and for the interaction lists of up to 49,152 target groups (and of the
+     * longest groups of larger solves) a pool of 0.2 GB for 1,000 groups, 0.5 GB for 4,000 and at most 0.8 GB. If less
+     * is free, the pool is what there is room for, down to some 10 MB, and the traversal takes more launches. The
+     * context keeps its scratch. The traverse and batched calls take the same pool. */
     RYO_API ryo_status ryo_solve_f32(ryo_ctx_t* ctx, const ryo_solve_params* params, float* x, float* y, float* z,
                                      float* m, float* h, float* vx, float* vy, float* vz, size_t n, float* p,
                                      float* ax, float* ay, float* az, uint32_t* order, ryo_solve_stats* stats,
@@ -555,7 +559,8 @@ extern "C"
     {
         ryo_solve_params solve; /* bucketSize, groupSize, theta, G, ewald, stackCapacity, timing */
         double hbmBudgetBytes;  /* admission budget (default 120e9) */
-        double bytesPerBody;    /* device bytes charged per resident body (default 256) */
+        double bytesPerBody;    /* device bytes charged per resident body (default 256); the lists' pool of the
+                                   solves (ryo_solve_f32) comes beside the budget */
         int maxSystems;         /* resident requests at most (default and upper limit RYO_BATCH_MAX_SYSTEMS) */
         uint64_t reserveBodies; /* resident bodies the arenas hold from creation on (default 0: grown on demand,
                                    doubling, which waits for the device at each growth) */

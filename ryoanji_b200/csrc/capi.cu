@@ -582,7 +582,8 @@ constexpr int kDepthFirst = 128;
 // the largest stack capacities accepted, for float and double coordinates: four warps' stacks beside the fused kernels'
 // staging in 227 KB of shared memory. No walk needs more than kMaxStackCapacity, which all kernels have room for.
 constexpr int kMostCapacity = 12344, kMostCapacity64 = 13120;
-constexpr size_t kListBytes     = size_t(512) << 20; // of list items
+constexpr size_t kListBytes     = size_t(512) << 20; // of list words; an item has 2 KB of sums beside its words
+constexpr uint32_t kLeastItems  = 1024;
 // interactions of an item: half the groups' number, at least 1024 (16 evaluation batches), below 512 groups twice their
 // number, so that the items of the smallest solves still number as many as the GPU has warps: 1,000 bodies 303 -> 267
 // us, the traversal of 4,096 bodies 105 -> 95 us, of 16,384 bodies 203 -> 193 us. Four times their number is slower
@@ -618,6 +619,31 @@ void readControl(ryo_ctx* ctx, Control& c, cudaStream_t s)
     c = ctx->results->ctl;
 }
 
+/*! the lists' pool of t.itemCapacity items, or of half as many, and so on down to @p least, if the memory has no room for
+ *  them: the traversal then takes more launches. What a context once found too large it does not ask for again. */
+void listPool(ryo_ctx* ctx, TraverseLaunch& t, uint32_t least, cudaStream_t s)
+{
+    while (true)
+    {
+        try
+        {
+            t.items    = ctx->scratch<ListItem>("trav.items", t.itemCapacity, s);
+            t.lists    = ctx->scratch<uint32_t>("trav.lists", size_t(t.itemCapacity) * t.itemWords, s);
+            t.partials = ctx->scratch<double4>("trav.partials", size_t(t.itemCapacity) * 2 * kWarp, s);
+            return;
+        }
+        catch (const CudaError& e)
+        {
+            if (e.err != cudaErrorMemoryAllocation || t.itemCapacity / 2 < least) throw;
+            cudaGetLastError(); // the next launch is not to find it
+            for (const char* name : {"trav.items", "trav.lists", "trav.partials"})
+                ctx->drop(name);
+            t.itemCapacity /= 2;
+            ctx->listLimit = t.itemCapacity;
+        }
+    }
+}
+
 /*! traverses t's groups, or those of @p list, through interaction lists until every group has been served or has
  *  overflowed the stack. Lists are cut by the solve's group count and the walk alone, so a group's sums do not depend
  *  on the launch or pass that it falls in. */
@@ -634,22 +660,23 @@ void traverseLists(ryo_ctx* ctx, TraverseLaunch t, const uint32_t* list, uint32_
     t.itemCost  = std::min(kMaxItemCost, std::max(minCost, solveGroups / 2));
     t.itemWords = t.subWalks > 1 ? 512 : 2048;
     const size_t tasks = size_t(count) * t.subWalks;
-    // pieces per part of a walk seldom pass this; when they do, the groups that found no room walk again
-    const size_t pieces = (t.subWalks > 1 ? 6 : 3) * tasks;
+    // A task's pieces seldom pass this; when they do, the groups that found no room walk again. At theta 0.5 and 0.4 a
+    // part has 1.2 to 2.6 pieces and a whole walk 1 to 3.5; at 0.2 parts of up to 2,048 groups have about five.
+    const size_t pieces = (t.subWalks > 1 && solveGroups <= 2048 ? 6 : 3) * tasks;
     t.itemCapacity      = uint32_t(std::min(pieces, kListBytes / (t.itemWords * sizeof(uint32_t))) + 4096);
-    t.taskLast          = ctx->scratch<int>("trav.taskLast", tasks, s);
-    t.groupState        = ctx->scratch<uint32_t>("trav.groupState", 3 * size_t(numGroups), s);
-    t.countM2P          = t.groupState + numGroups;
-    t.countP2P          = t.countM2P + numGroups;
+    if (ctx->listLimit > 0) t.itemCapacity = std::min(t.itemCapacity, ctx->listLimit);
+    t.taskLast   = ctx->scratch<int>("trav.taskLast", tasks, s);
+    t.groupState = ctx->scratch<uint32_t>("trav.groupState", 3 * size_t(numGroups), s);
+    t.countM2P   = t.groupState + numGroups;
+    t.countP2P   = t.countM2P + numGroups;
     RYO_CUDA(cudaMemsetAsync(t.groupState, 0, 3 * sizeof(uint32_t) * size_t(numGroups), s));
     uint32_t* unserved[2] = {ctx->scratch<uint32_t>("trav.unservedA", count, s),
                              ctx->scratch<uint32_t>("trav.unservedB", count, s)};
     uint32_t chunk = count; // groups per launch
+    uint32_t least = kLeastItems;
     for (int flip = 0;; flip ^= 1)
     {
-        t.items      = ctx->scratch<ListItem>("trav.items", t.itemCapacity, s);
-        t.lists      = ctx->scratch<uint32_t>("trav.lists", size_t(t.itemCapacity) * t.itemWords, s);
-        t.partials   = ctx->scratch<double4>("trav.partials", size_t(t.itemCapacity) * 2 * kWarp, s);
+        listPool(ctx, t, least, s);
         uint32_t left = 0;
         for (uint32_t first = 0; first < count; first += chunk)
         {
@@ -663,7 +690,11 @@ void traverseLists(ryo_ctx* ctx, TraverseLaunch t, const uint32_t* list, uint32_
         }
         if (left == 0) return;
         // groups that found no room walk again, fewer at a time; the pool grows only when it did not hold one group
-        if (chunk == 1) t.itemCapacity *= 4;
+        if (chunk == 1)
+        {
+            least = t.itemCapacity + 1;
+            t.itemCapacity *= 4;
+        }
         if (2 * left > count) chunk = std::max(1u, std::min(chunk, left) / 8);
         list  = unserved[flip];
         count = left;

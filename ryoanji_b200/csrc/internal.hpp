@@ -120,6 +120,7 @@ struct ryo_ctx
     cudaStream_t copyStream         = nullptr; // host solves: copies that overlap the solve
 
     HostResults* results = nullptr;
+    uint32_t listLimit   = 0; // items that the memory had room for when a traversal's lists found too little (0: never)
 
     struct Buffer
     {
@@ -153,6 +154,14 @@ struct ryo_ctx
             b.bytes = grow;
         }
         return static_cast<T*>(b.ptr);
+    }
+
+    void drop(const std::string& name)
+    {
+        auto it = buffers.find(name);
+        if (it == buffers.end()) return;
+        if (it->second.ptr) RYO_CUDA(cudaFree(it->second.ptr)); // waits for the device
+        buffers.erase(it);
     }
 
     void releaseAll()
