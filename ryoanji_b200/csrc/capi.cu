@@ -31,6 +31,7 @@ struct ApiError
 ryo_status fromCuda(const CudaError& e, std::string& msg)
 {
     msg = std::string(e.what) + ": " + cudaGetErrorString(e.err);
+    cudaGetLastError(); // reported here: the next call's first launch is not to find it
     if (e.err == cudaErrorMemoryAllocation) return RYO_ERR_OOM;
     if (e.err == cudaErrorInvalidValue) return RYO_ERR_BAD_ARG;
     if (e.err == cudaErrorNoDevice || e.err == cudaErrorInvalidDevice) return RYO_ERR_NO_DEVICE;

@@ -386,6 +386,7 @@ ryo_status engineGuard(ryo_engine* E, const std::function<void()>& f)
     catch (const CudaError& e)
     {
         E->lastError = std::string(e.what) + ": " + cudaGetErrorString(e.err);
+        cudaGetLastError(); // reported here
         return e.err == cudaErrorMemoryAllocation ? RYO_ERR_OOM : RYO_ERR_CUDA;
     }
     catch (const std::bad_alloc&)
@@ -452,6 +453,7 @@ extern "C" ryo_status ryo_engine_create(ryo_ctx_t* ctx, const ryo_engine_params*
     catch (const CudaError& e)
     {
         ctx->lastError = std::string("engine_create: ") + e.what + ": " + cudaGetErrorString(e.err);
+        cudaGetLastError(); // reported here
         delete E;
         return e.err == cudaErrorMemoryAllocation ? RYO_ERR_OOM : RYO_ERR_CUDA;
     }

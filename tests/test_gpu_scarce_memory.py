@@ -1,5 +1,5 @@
 """Traversals whose interaction lists find too little free memory take what there is, in more launches, with the same
-bits."""
+bits; and a call that fails for lack of memory leaves no error behind."""
 import numpy as np
 import pytest
 import torch
@@ -88,3 +88,22 @@ def test_double_traversal_with_little_memory(real):
         del hog
         torch.cuda.empty_cache()
     assert torch.equal(got, base) and s == stats
+
+def test_failed_allocation_leaves_no_error():
+    import ryoanji_b200 as ryo
+    n = 1 << 22
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(1)
+    bodies = [torch.rand(n, generator=gen, device="cuda") for _ in range(4)] + [torch.full((n,), 1e-4, device="cuda")]
+    work, out = [b.clone() for b in bodies], torch.empty(4, n, device="cuda")
+    ctx = ryo.Context()
+    hog = _fill(96 << 20)  # the sort alone of four million bodies takes more
+    try:
+        with pytest.raises(ryo.RyoError) as e:
+            _solve(ryo, bodies, work, out, ryo.SolveParams(), ctx)
+        assert e.value.status == 3
+    finally:
+        del hog
+        torch.cuda.empty_cache()
+    _solve(ryo, bodies, work, out, ryo.SolveParams(), ctx)
+    assert torch.isfinite(out).all()
