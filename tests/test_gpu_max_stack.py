@@ -125,3 +125,20 @@ def test_depth_of_double_traversals(real, n):
     run(512)
     for k in (1, -1):  # the depth's own capacity, and the default's size given
         assert all(torch.equal(a, b) for a, b in zip(results[0], results[k]))
+
+
+def test_depth_of_a_batch():
+    import ryoanji_b200 as ryo
+    from ryoanji_b200 import datasets as ds
+    sets = [ds.plummer(3001, seed=1, velocities=False), ds.periodic_box(2000, seed=2, eps=0.002),
+            ds.plummer(70, seed=3, velocities=False), ds.periodic_box(9000, seed=4, eps=0.002)]
+    bodies = [torch.cat([dev(getattr(p, k)) for p in sets]) for k in ("x", "y", "z", "m", "h")]
+    systems = [ryo.BatchSystem(p.n, ryo.Box(*p.box, boundary=(ryo.BOUNDARY_PERIODIC,) * 3) if i % 2 else None, 2)
+               for i, p in enumerate(sets)]
+
+    def run(capacity):
+        out = torch.empty(4, bodies[0].numel(), device="cuda")
+        r = ryo.solve_batch(systems, *(b.clone() for b in bodies), *out,
+                            params=ryo.SolveParams(theta=0.5, bucket_size=32, stack_capacity=capacity)).stats
+        return r.max_stack, r.retries, (r.sum_p2p, r.max_p2p, r.sum_m2p, r.max_m2p)
+    _tight(run)
