@@ -631,8 +631,9 @@ template<class Kernel>
 unsigned residentBlocks(Kernel kernel, size_t smem, size_t warps, int smCount)
 {
     int perSm = 0;
+    // the limit is the kernel's, for all threads and contexts: always the same value, with room for the deepest stacks
     if (smem > 48 * 1024)
-        RYO_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+        RYO_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024));
     RYO_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, kernel, kTravThreads, smem));
     return unsigned(std::min((warps + kTravWarps - 1) / kTravWarps, size_t(std::max(perSm, 1)) * smCount));
 }

@@ -736,14 +736,9 @@ static void launchTyped64(const TraverseLaunch& t, int smCount, cudaStream_t s)
         return;
     }
     auto kernel = t.mdqArrays ? traverseKernel64<true, Th, Tm, Ta, Tmp> : traverseKernel64<false, Th, Tm, Ta, Tmp>;
+    static_assert(kT64Threads == kTravThreads);
     size_t smem = sizeof(WarpSmem64) * kT64Warps + sizeof(int) * kT64Warps * size_t(t.stackCapacity);
-    RYO_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
-    int perSm = 0;
-    RYO_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, kernel, kT64Threads, smem));
-    if (perSm < 1) perSm = 1;
-    int want   = (t.numGroups + kT64Warps - 1) / kT64Warps;
-    int blocks = min(want, perSm * smCount);
-    kernel<<<blocks, kT64Threads, smem, s>>>(t, A);
+    kernel<<<residentBlocks(kernel, smem, size_t(t.numGroups), smCount), kT64Threads, smem, s>>>(t, A);
     RYO_LAUNCH_CHECK();
 }
 
