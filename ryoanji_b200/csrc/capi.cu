@@ -572,9 +572,29 @@ __global__ void splitGroupsKernel(const __grid_constant__ TraverseLaunch t, uint
 }
 
 /*! groups up to which a traversal goes through interaction lists: walks first, then the evaluation of list pieces of
- *  similar cost by all warps. Larger ones keep the GPU busy with a group per warp, which saves the lists' traffic. */
-constexpr uint32_t kListGroups  = 49152;
-constexpr uint32_t kSubGroups   = 6000;  // groups up to which every list walk is split into eight parts
+ *  similar cost by all warps. Larger ones keep the GPU busy with a group per warp, which saves the lists' traffic.
+ *  Traversal in ms, lists against fused kernel, at bucket 64 and theta 0.5 unless said:
+ *  - open float systems: Plummer 12,000 groups 5.35 and 6.33, 16,384 6.78 and 7.07, 20,000 8.70 and 8.59, 45,000 17.8
+ *    and 16.7; eight halos 16,384 5.45 and 6.68, 36,000 12.45 and 12.56; cube 12,000 2.22 and 2.15, 45,000 7.57 and 7.22.
+ *  - periodic ones, whose groups are alike and whose lists are long: box 2,000 0.70 and 0.72, 4,096 1.39 and 1.32, 6,000
+ *    1.77 and 1.57, but 16,384 4.73 and 4.93; at theta 0.4 and bucket 16 3,000 1.34 and 1.25, 16,384 7.13 and 6.09; a
+ *    Plummer sphere in a third of the box's bodies there 2,000 1.21 and 1.31, 8,000 6.55 and 3.94.
+ *  - batches, whose largest systems hold the longest groups: 2^10 to 2^15 bodies 30,000 5.70 and 6.38, 48,824 8.93 and
+ *    9.38; systems of up to 2^13 only 49,057 5.33 and 5.16.
+ *  - double coordinates, without queue for long groups in the fused kernel: cube 45,000 14.7 and 15.3, Plummer 16,384
+ *    13.5 and 20.0, 45,000 34.5 and 35.1; with replicas cube 16,384 8.56 and 9.42, Plummer 32,768 34.9 and 32.6. */
+uint32_t listGroups(const TraverseLaunch& t)
+{
+    const bool replicas = t.numShells > 0;
+    if (t.precision != kPrecisionF32) return replicas ? 24576 : 49152;
+    if (t.groupSys) return 49152;
+    return replicas ? 2560 : 16384;
+}
+
+//! groups up to which every list walk is split into eight parts, so that the longest walk does not hold up the rest.
+//! Traversal in ms, parts against whole walks: Plummer 5,000 groups 2.33 and 4.29, 6,000 2.66 and 2.77, 7,000 3.18 and
+//! 3.11; cube 2,000 0.44 and 0.50, 4,000 0.89 and 0.81, 6,000 1.08 and 0.99.
+constexpr uint32_t kSubGroups = 6000;
 // stack capacities below which divided walks have their depths taken before them. Open and periodic solves hold up to
 // about 110 entries, so below that groups may fail, whose lists and sums would be for nothing (250,000 bodies of a
 // cube, a capacity of 6 entries: 16.7 -> 4.9 ms); where all fit, it costs the longest walk's time (60,001 Plummer
@@ -592,7 +612,9 @@ constexpr uint32_t kLeastItems  = 1024;
 // same alone and among others.
 constexpr unsigned kMinItemCost = 1024;
 constexpr unsigned kMaxItemCost = 16384;
-constexpr unsigned kHeavyCost   = 32768; // of the fused kernel's groups; compact ones cost about 17,000 at most
+// cost past which the fused kernel queues a group for the lists; compact groups cost about 17,000 at most. Below 11,840
+// groups, four per resident warp, the longest group shows and the line falls with their number, to half of it.
+constexpr unsigned kHeavyCost = 32768, kHeavyGroups = 11840;
 
 /*! the groups of a traverse call are the caller's: each must hold 1 to 64 targets inside [firstBody, lastBody). A
  *  warp evaluates at most 64 targets, and an empty group would read before its start. The reference refuses
@@ -727,13 +749,14 @@ void runTraversal(ryo_ctx* ctx, TraverseLaunch t, cudaStream_t s, double* potent
     {
         if (pass > 0) launchTraversalReset(ctx->ctl, kTravPass, s);
         ++pass;
-        if (solveGroups <= kListGroups)
+        if (solveGroups <= listGroups(t))
             traverseLists(ctx, t, nullptr, uint32_t(t.numGroups), solveGroups, hc, s);
         else
         {
             t.heavyGroups   = ctx->scratch<uint32_t>("trav.heavy", std::max(t.numGroups, 1), s);
             t.heavyCapacity = uint32_t(t.numGroups);
-            t.heavyCost     = kHeavyCost;
+            t.heavyCost     = unsigned(std::clamp(uint64_t(kHeavyCost) * solveGroups / kHeavyGroups,
+                                                  uint64_t(kHeavyCost / 2), uint64_t(kHeavyCost)));
             launchTraverse(t, ctx->smCount, s);
             readControl(ctx, hc, s);
             if (hc.heavyCount > 0)
