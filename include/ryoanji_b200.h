@@ -289,7 +289,9 @@ extern "C"
     {
         uint32_t* groupM2P; /* device, numGroups entries (may be NULL): approximated cells per group */
         uint32_t* groupP2P; /* device, numGroups entries (may be NULL): directly summed source bodies per group */
-        int stackCapacity;  /* traversal stack entries per warp, 0 = default (512); small values force splits */
+        int stackCapacity;  /* traversal stack entries per warp, 0 = default (512); small values force splits. A
+                               capacity of the reported maxStack never does; no result depends on one that fits. At
+                               most 12,344, or 13,120 for double coordinates (RYO_ERR_BAD_ARG otherwise) */
         int multipole;      /* RYO_MULTIPOLE_QUADRUPOLE: 8 floats per node in multipoles (default);
                                RYO_MULTIPOLE_MDQ: 12 floats per node (CartesianMDQpole, traversal_gpu.cu:641) */
     } ryo_traverse_options;
@@ -309,7 +311,8 @@ extern "C"
      * float, Tf = double, multipoles of floats), the caller side of codes whose particle positions are double. As in
      * the reference, the MAC and the sums run in double with the single-precision rsqrt of the double argument
      * (kernel.hpp:38-52). Centres are 4 doubles per node; multipoles 8 values per node, or 12 with options->multipole
-     * = RYO_MULTIPOLE_MDQ. Semantics, checks and statistics are those of ryo_traverse_ex_f32 (options may be NULL). */
+     * = RYO_MULTIPOLE_MDQ. Semantics, checks and statistics are those of ryo_traverse_ex_f32 (options may be NULL).
+     * Above 49,152 groups (24,576 with replicas) a group too costly for one warp is evaluated by one warp here. */
     RYO_API ryo_status ryo_traverse_f64(ryo_ctx_t* ctx, const ryo_group_view* grp, int initNodeIdx, const double* xt,
                                         const double* yt, const double* zt, const double* mt, const double* ht,
                                         const double* xs, const double* ys, const double* zs, const double* ms,
@@ -495,9 +498,9 @@ extern "C"
     /* x, y, z, m, h: in any order on entry, SFC-sorted on return; vx, vy, vz (may be NULL) are permuted along;
      * p, ax, ay, az are overwritten with the potential (G m phi) and acceleration in sorted order; order (may be
      * NULL) receives the original index of each sorted body. stats (host, may be NULL).
-     * Device scratch: about 130 bytes per body, and for the interaction lists of up to 49,152 target groups (and of the
-     * longest groups of larger solves) a pool of 0.2 GB for 1,000 groups, 0.5 GB for 4,000 and at most 0.8 GB. If less
-     * is free, the pool is what there is room for, down to some 10 MB, and the traversal takes more launches. The
+     * Device scratch: about 130 bytes per body, and for the interaction lists of up to 16,384 target groups (2,560 in a
+     * periodic box; of the longest groups of larger solves too) a pool of 0.2 GB for 1,000 groups, 0.5 GB for 4,000 and
+     * at most 0.8 GB. If less is free, the pool is what there is room for, down to some 10 MB, and the traversal takes more launches. The
      * context keeps its scratch. The traverse and batched calls take the same pool. */
     RYO_API ryo_status ryo_solve_f32(ryo_ctx_t* ctx, const ryo_solve_params* params, float* x, float* y, float* z,
                                      float* m, float* h, float* vx, float* vy, float* vz, size_t n, float* p,

@@ -98,7 +98,8 @@ static void launchBatchRanges(const float* a0, const float* a1, const float* a2,
 {
     if (n == 0) return;
     // at most about 64 warps per SM, so that few atomics meet at a large system's values
-    const size_t rounds = (n + size_t(kRangeStep) * 9472 - 1) / (size_t(kRangeStep) * 9472);
+    const size_t most   = size_t(kRangeStep) * 64 * 148;
+    const size_t rounds = (n + most - 1) / most;
     const size_t chunk  = rounds * kRangeStep;
     const size_t warps  = (n + chunk - 1) / chunk;
     batchRangesKernel<kArrays, kSkipNaN><<<ceilDiv(warps * kWarp, 128), 128, 0, s>>>(a0, a1, a2, n, chunk, first,

@@ -608,8 +608,8 @@ constexpr uint32_t kLeastItems  = 1024;
 // interactions of an item: half the groups' number, at least 1024 (16 evaluation batches), below 512 groups twice their
 // number, so that the items of the smallest solves still number as many as the GPU has warps: 1,000 bodies 303 -> 267
 // us, the traversal of 4,096 bodies 105 -> 95 us, of 16,384 bodies 203 -> 193 us. Four times their number is slower
-// between 128 and 512 groups (16,384 bodies 202 us). A batched solve keeps 1024, so that a small system's sums are the
-// same alone and among others.
+// between 128 and 512 groups (16,384 bodies 202 us). A batched solve keeps at least 1024, however few its groups: a
+// system's lists are then cut alike in every batch of up to 2,048 groups, from itself alone on.
 constexpr unsigned kMinItemCost = 1024;
 constexpr unsigned kMaxItemCost = 16384;
 // cost past which the fused kernel queues a group for the lists; compact groups cost about 17,000 at most. Below 11,840

@@ -260,7 +260,7 @@ static void launchDirectPacked(size_t first, size_t last, size_t numBodies, cons
     // of sources; up to nine per SM are resident, so that a little more than eight still runs as one wave
     const unsigned blocks = ceilDiv(last - first, kPackedTargets);
     unsigned splits       = 1;
-    while (splits < unsigned(kMaxSplit) && blocks * splits < 1184 && numBodies / (2 * splits) >= kPackedTile)
+    while (splits < unsigned(kMaxSplit) && blocks * splits < 8 * 148 && numBodies / (2 * splits) >= kPackedTile)
         splits *= 2;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim  = dim3(blocks * splits);

@@ -14,9 +14,9 @@
  *     warp, go through interaction lists: walkKernel writes each group's cells and direct leaves to pieces of bounded
  *     cost, evalKernel evaluates the pieces in any order, finishKernel adds them up. A solve's time is then no longer
  *     that of its longest group. Traversal of a Plummer sphere of 60,001 bodies (938 groups, the longest seven times
- *     the mean): 0.48 ms, against 1.24 ms by the fused kernel with its longest groups repeated by several warps; of
- *     2^20 bodies: 6.8 against 7.4 ms; of 256 batched spheres (42,002 groups): 8.2 against 8.9 ms. From about 50,000
- *     groups the fused kernel is as fast and needs no lists;
+ *     the mean): 0.49 ms, against 1.24 ms by the fused kernel with its longest groups repeated by several warps; of
+ *     2^20 bodies: 6.8 against 7.4 ms; of 256 batched spheres (42,002 groups): 8.3 against 8.9 ms. The group counts at
+ *     which lists stop paying stand at the rule (capi.cu, listGroups);
  *   - depth-first traversal over a per-warp stack in shared memory (entries are the first of eight siblings;
  *     four entries, 32 cells, are tested per step), bounded by the stack capacity; a group that would exceed it is
  *     reported and split by the host, as the reference does with its global queue;

@@ -17,10 +17,10 @@
  * trades that rate for the callers' precision.
  *
  * As in float, launches of few groups go through interaction lists (lists.cuh) and larger ones through the fused
- * kernel. The list evaluation is bound by the FP64 pipe (13 operations, 26 cycles, per direct pair and sub-core; the
- * pipe is 70% busy) and the latency of its chains beside the conversions around rsqrt: it leaves the softening's
- * maximum out where a batch lies beyond it, runs four sources of two targets at once, and reads staged cells 16 bytes
- * at a time. The step flow of 120,001 Plummer bodies, everything double: 2.3 ms per pass, against 6.3 ms with the
+ * kernel, which here does not queue long groups. The list evaluation is bound by the FP64 pipe (13 operations, 26
+ * cycles, per direct pair and sub-core; the pipe is 70% busy) and the latency of its chains beside the conversions
+ * around rsqrt: it leaves the softening's maximum out where a batch lies beyond it, runs four sources of two targets at
+ * once, and reads staged cells 16 bytes at a time. The step flow of 120,001 Plummer bodies, everything double: 2.3 ms per pass, against 6.3 ms with the
  * fused kernel (whose time is its longest group's); 250,000 bodies of a cube, float masses: 2.44 against 2.80 ms. Its
  * evaluation takes 1.26 and 1.39 ms (two sources at once 1.32 and 1.53 ms, five blocks per SM 1.33 and 1.52 ms, cells
  * read 8 bytes at a time from stages that share their banks 1.28 and 1.44 ms).
