@@ -8,7 +8,7 @@
  * What bounds it: the walk of many groups is bound by instruction issue and the L1 (a step of 32 cells takes about 170
  * instructions with the list's writing; 5% of the evaluation's time), that of few groups by the latency of its longest
  * part. The parts of a divided walk load two steps' cells at once: 60,001 Plummer bodies 132 -> 112 us. A whole walk
- * does not, which costs it up to a fifth of its time (2^20 bodies 398 against 338 us, 1% of the solve): it is the walk
+ * does not, which costs it up to a fifth of its time (2^20 bodies 430 against 340 us, 1% of the solve): it is the walk
  * whose depth the caller sees. Divided ones have theirs taken beside the evaluation (walkDepth), at 1 to 3% of a solve.
  * The lists take 6-15 KB per group and stay in the L2 between the two kernels.
  */
@@ -659,8 +659,9 @@ template<class Sink>
 void launchFinish(const TraverseLaunch& t, const Sink& sink, int smCount, cudaStream_t s)
 {
     // a block per group for as many groups as two rounds of eight blocks per SM take: the chains are long there
-    // (100,003 bodies at theta 0.2, 1,563 groups: 81 -> 22 us; 60,001 Plummer bodies: 32 -> 17 us), but with 3,907
-    // groups of a cube, whose parts are an item or two, it took 34 instead of 20 us
+    // (100,003 bodies at theta 0.2, 1,563 groups: 81 -> 22 us, and 45 us since the items' sums are doubles; 60,001
+    // Plummer bodies: 32 -> 17 us, now 21), but with 3,907 groups of a cube, whose parts are an item or two, it took 34
+    // instead of 20 us
     const size_t numGroups = size_t(t.numGroups);
     if (t.subWalks == kWalkParts && numGroups <= size_t(16) * smCount)
         finishKernel<true><<<unsigned(std::min(numGroups, size_t(8) * smCount)), kFinishThreads, 0, s>>>(t, sink);

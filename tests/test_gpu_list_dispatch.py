@@ -7,7 +7,7 @@ import torch
 pytestmark = pytest.mark.gpu
 
 
-def _tree(kind, n, shells):
+def _tree(kind, n, shells, special=None):
     import ryoanji_b200 as ryo
     ct = torch.float32 if kind == "f32" else torch.float64
     rt = torch.float64 if kind == "f64" else torch.float32
@@ -16,6 +16,8 @@ def _tree(kind, n, shells):
     x, y, z = (torch.from_numpy(np.ascontiguousarray(v)).cuda().to(ct) for v in p.T)
     m = torch.from_numpy(rng.uniform(0.5, 1.5, n) / n).cuda().to(rt)
     h = torch.full((n,), 1e-3, device="cuda", dtype=rt)
+    if special:
+        {"m": m, "h": h}[special[0]][n // 3] = special[1]
     tb, box = ryo.TreeBuilder(32), ryo.Box.cube(-1.0, 1.0)
     nn = tb.update(x, y, z, box)
     centers = torch.zeros(nn, 4, device="cuda", dtype=ct)
@@ -52,3 +54,21 @@ def test_both_sides_agree(kind, shells, last):
     assert np.percentile(err, 99) < bound[0] and err.max() < bound[1]
     assert torch.allclose(a[0], b[0], rtol=10 * bound[0], atol=float(a[0].abs().max()) * bound[0])
     assert abs(fused[4] - lists[4]) <= 64  # the pair may walk deeper than either of its bodies
+
+
+# (a mass of NaN or infinity makes every body's sums NaN or infinite; a softening only its own pairs')
+@pytest.mark.parametrize("special", [("m", np.nan), ("m", np.inf), ("h", np.nan), ("h", np.inf), ("h", -1e-3)])
+@pytest.mark.parametrize("kind,shells,last", [("f32", 0, 16384), ("f32", 1, 2560), ("f64", 0, 49152),
+                                              ("mixed", 1, 24576)])
+def test_special_values(kind, shells, last, special):
+    n = last + 1
+    run = _tree(kind, n, shells, special)
+    ones = torch.arange(n + 1, device="cuda", dtype=torch.int32)
+    fused, lists = run(ones), run(torch.cat([ones[:n - 1], ones[n:]]))
+    a, b = fused[0][:, :n - 2], lists[0][:, :n - 2]
+    assert torch.equal(a.isnan(), b.isnan())
+    inf = a.isinf()
+    assert torch.equal(inf, b.isinf()) and torch.equal(a[inf], b[inf])
+    ok = a.isfinite()
+    if ok.any():
+        assert float((a - b)[ok].abs().max()) <= 1e-5 * float(a[ok].abs().max())
