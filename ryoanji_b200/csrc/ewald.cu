@@ -128,14 +128,18 @@ __global__ void ewaldKernel(const __grid_constant__ EwaldKernelParams<R> E, cons
                             const Tc* __restrict__ y, const Tc* __restrict__ z, const Tm* __restrict__ m, float G,
                             Ta* ugrav, Ta* ax, Ta* ay, Ta* az, double* potential)
 {
-    // from 2^26 groups on the threads' numbers pass 32 bits
-    const size_t warpGlobal = (size_t(blockIdx.x) * blockDim.x + threadIdx.x) / kWarp;
-    const int lane          = laneId();
-    double upot             = 0.0;
-    if (warpGlobal / 2 < numGroups)
+    // the first half of the blocks takes the first 32 targets of the groups, the second half the others, so that blocks
+    // without any leave at once: 60,000 targets in groups of 32, double, 186 us, against 247 us with a group's two warps
+    // side by side, 198 us with one warp, and 185 us in groups of 64 either way. From 2^26 groups on the threads' numbers
+    // pass 32 bits.
+    const unsigned half = blockIdx.x >= gridDim.x / 2 ? 1 : 0;
+    const size_t group  = size_t(blockIdx.x - half * (gridDim.x / 2)) * (blockDim.x / kWarp) + threadIdx.x / kWarp;
+    const int lane      = laneId();
+    double upot         = 0.0;
+    if (group < numGroups)
     {
-        uint32_t b = groupStart[warpGlobal / 2], e = groupEnd[warpGlobal / 2];
-        for (size_t i = b + (warpGlobal & 1) * kWarp + lane; i < e; i += 2 * kWarp)
+        uint32_t b = groupStart[group], e = groupEnd[group];
+        for (size_t i = b + half * kWarp + lane; i < e; i += 2 * kWarp)
         {
             R pos[3]  = {R(x[i]), R(y[i]), R(z[i])};
             R acc[4]  = {E.k1 * E.mroot[0], R(0), R(0), R(0)};
@@ -277,7 +281,7 @@ static void launchEwaldTyped(const EwaldHost& h, const uint32_t* groupStart, con
         E.fc2[E.numK++] = 2 * k[3];
     }
     unsigned threads = 128;
-    unsigned blocks  = ceilDiv(size_t(numGroups) * 2 * kWarp, threads);
+    unsigned blocks  = 2 * ceilDiv(size_t(numGroups) * kWarp, threads);
     ewaldKernel<R, Tc, Tm, Ta><<<blocks, threads, 0, s>>>(E, groupStart, groupEnd, numGroups, x, y, z, m, G, ugrav,
                                                            ax, ay, az, potentialOut);
     RYO_LAUNCH_CHECK();
