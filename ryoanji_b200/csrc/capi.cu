@@ -578,7 +578,8 @@ __global__ void splitGroupsKernel(const __grid_constant__ TraverseLaunch t, uint
  *    and 16.7; eight halos 16,384 5.45 and 6.68, 36,000 12.45 and 12.56; cube 12,000 2.22 and 2.15, 45,000 7.57 and 7.22.
  *  - periodic ones, whose groups are alike and whose lists are long: box 2,000 0.70 and 0.72, 4,096 1.39 and 1.32, 6,000
  *    1.77 and 1.57, but 16,384 4.73 and 4.93; at theta 0.4 and bucket 16 3,000 1.34 and 1.25, 16,384 7.13 and 6.09; a
- *    Plummer sphere in a third of the box's bodies there 2,000 1.21 and 1.31, 8,000 6.55 and 3.94.
+ *    Plummer sphere with a third of the bodies around it there 2,000 1.21 and 1.31, 8,000 6.55 and 3.94. (A set far
+ *    from its images is the other way round: a cube in a box twice its side 3,125 1.00 and 1.58.)
  *  - batches, whose largest systems hold the longest groups: 2^10 to 2^15 bodies 30,000 5.70 and 6.38, 48,824 8.93 and
  *    9.38; systems of up to 2^13 only 49,057 5.33 and 5.16.
  *  - double coordinates, without queue for long groups in the fused kernel: cube 45,000 14.7 and 15.3, Plummer 16,384
@@ -613,8 +614,9 @@ constexpr uint32_t kLeastItems  = 1024;
 constexpr unsigned kMinItemCost = 1024;
 constexpr unsigned kMaxItemCost = 16384;
 // cost past which the fused kernel queues a group for the lists; compact groups cost about 17,000 at most. Below 11,840
-// groups, four per resident warp, the longest group shows and the line falls with their number, to half of it.
-constexpr unsigned kHeavyCost = 32768, kHeavyGroups = 11840;
+// groups, four per resident warp, the longest group shows and the line falls with their number. At 8,192 it would meet
+// ordinary groups (3,000 groups of a periodic box at theta 0.4, bucket 16: 1.58 ms, and 1.24 ms at 12,288).
+constexpr unsigned kHeavyCost = 32768, kLeastHeavyCost = 12288, kHeavyGroups = 11840;
 
 /*! the groups of a traverse call are the caller's: each must hold 1 to 64 targets inside [firstBody, lastBody). A
  *  warp evaluates at most 64 targets, and an empty group would read before its start. The reference refuses
@@ -756,7 +758,7 @@ void runTraversal(ryo_ctx* ctx, TraverseLaunch t, cudaStream_t s, double* potent
             t.heavyGroups   = ctx->scratch<uint32_t>("trav.heavy", std::max(t.numGroups, 1), s);
             t.heavyCapacity = uint32_t(t.numGroups);
             t.heavyCost     = unsigned(std::clamp(uint64_t(kHeavyCost) * solveGroups / kHeavyGroups,
-                                                  uint64_t(kHeavyCost / 2), uint64_t(kHeavyCost)));
+                                                  uint64_t(kLeastHeavyCost), uint64_t(kHeavyCost)));
             launchTraverse(t, ctx->smCount, s);
             readControl(ctx, hc, s);
             if (hc.heavyCount > 0)

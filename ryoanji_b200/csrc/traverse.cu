@@ -625,24 +625,13 @@ __device__ __forceinline__ int evalP2P(WarpSmem& S, int numLeaves, bool all, con
     return keep;
 }
 
-/*! the fused kernel's evaluations. With dipoles they are calls: inlined four times the kernel's code is so long that a
- *  traversal of 3.3M Plummer bodies takes 25.4 instead of 23.5 ms. Without, inlining is as fast or faster (4M bodies of a
- *  cube 10.6 and 10.9 ms), as it is in evalKernel. */
-template<class Nodes>
-__device__ __noinline__ void callM2P(WarpSmem& S, int count, const Nodes& nodes, const TargetState& T)
-{
-    evalM2P(S, 0, count, nodes, T);
-}
+/*! the fused kernel's direct sums. With dipoles they are a call: inlined twice beside the long cell loops they slow a
+ *  traversal of 3.3M Plummer bodies from 23.3 to 25.4 ms. Without, inlining is as fast or faster (4M bodies of a cube 10.6
+ *  and 10.9 ms), as it is in evalKernel. */
 template<class Sources>
 __device__ __noinline__ int callP2P(WarpSmem& S, int numLeaves, bool all, const Sources& src, const TargetState& T)
 {
     return evalP2P(S, numLeaves, all, src, T);
-}
-template<class Nodes>
-__device__ __forceinline__ void fusedM2P(WarpSmem& S, int count, const Nodes& nodes, const TargetState& T)
-{
-    if constexpr (Nodes::kDipole) callM2P(S, count, nodes, T);
-    else evalM2P(S, 0, count, nodes, T);
 }
 template<class Nodes, class Sources>
 __device__ __forceinline__ int fusedP2P(WarpSmem& S, int numLeaves, bool all, const Sources& src, const TargetState& T)
@@ -901,7 +890,7 @@ __global__ void __launch_bounds__(kTravThreads, 5)
                         constexpr int kMB = m2pBatch<Nodes>();
                         while (nM >= kMB)
                         {
-                            fusedM2P(S, kMB, nodes, T);
+                            evalM2P(S, 0, kMB, nodes, T);
                             nM -= kMB; // fewer than kWarp cells remain: one move per lane
                             if (lane < nM) S.m2p[lane] = S.m2p[kMB + lane];
                             __syncwarp();
@@ -910,7 +899,7 @@ __global__ void __launch_bounds__(kTravThreads, 5)
                     }
                     if (!overflow)
                     {
-                        if (nM > 0) fusedM2P(S, nM, nodes, T);
+                        if (nM > 0) evalM2P(S, 0, nM, nodes, T);
                         if (nL > 0) fusedP2P<Nodes>(S, nL, true, src, T);
                     }
 #pragma unroll
