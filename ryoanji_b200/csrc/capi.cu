@@ -686,8 +686,9 @@ void traverseLists(ryo_ctx* ctx, TraverseLaunch t, const uint32_t* list, uint32_
     t.itemWords = t.subWalks > 1 ? 512 : 2048;
     const size_t tasks = size_t(count) * t.subWalks;
     // A task's pieces seldom pass this; when they do, the groups that found no room walk again. At theta 0.5 and 0.4 a
-    // part has 1.2 to 2.6 pieces and a whole walk 1 to 3.5; at 0.2 parts of up to 2,048 groups have about five.
-    const size_t pieces = (t.subWalks > 1 && solveGroups <= 2048 ? 6 : 3) * tasks;
+    // part has 1.2 to 2.6 pieces and a whole walk 1 to 3.5; at 0.2 parts of up to 2,048 groups have about five, and so
+    // have those of queued groups (829 of a batch of 776,518 groups: 214 ms with room for three, 205 ms with six).
+    const size_t pieces = (t.subWalks > 1 && (list || solveGroups <= 2048) ? 6 : 3) * tasks;
     t.itemCapacity      = uint32_t(std::min(pieces, kListBytes / (t.itemWords * sizeof(uint32_t))) + 4096);
     if (ctx->listLimit > 0) t.itemCapacity = std::min(t.itemCapacity, ctx->listLimit);
     t.taskLast   = ctx->scratch<int>("trav.taskLast", tasks, s);
