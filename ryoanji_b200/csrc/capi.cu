@@ -613,7 +613,9 @@ constexpr uint32_t kLeastItems  = 1024;
 // system's lists are then cut alike in every batch of up to 2,048 groups, from itself alone on.
 constexpr unsigned kMinItemCost = 1024;
 constexpr unsigned kMaxItemCost = 16384;
-// cost past which the fused kernel queues a group for the lists; compact groups cost about 17,000 at most. Below 11,840
+// cost past which the fused kernel queues a group for the lists; compact groups cost about 17,000 at most at theta 0.5.
+// A lower line would suit eight halos (1.2M bodies 7.49 ms, 6.77 ms at 16,384) but meets every group at stricter angles
+// (1.2M Plummer bodies at theta 0.35: 16.6 ms, and 27.9 ms at 16,384, whose walks are made twice). Below 11,840
 // groups, four per resident warp, the longest group shows and the line falls with their number. At 8,192 it would meet
 // ordinary groups (3,000 groups of a periodic box at theta 0.4, bucket 16: 1.58 ms, and 1.24 ms at 12,288).
 constexpr unsigned kHeavyCost = 32768, kLeastHeavyCost = 12288, kHeavyGroups = 11840;
